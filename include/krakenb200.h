@@ -247,6 +247,16 @@ int kb_fused_natconv_vt_step(void *f_out, const void *f_in, void *g_out, const v
                              double alpha_visc, double omega_T, double beta_g, double T_ref_buoy,
                              double T_hot, double T_cold, int dtype, void *stream);
 
+/* One step of run_rayleigh_benard_2d (src/drivers/thermal.jl:101-130) in one
+ * launch, FP64 bits as the separate calls: stream f and g, two fixed-
+ * temperature faces, temperature, moments, thermal BGK, Boussinesq BGK.
+ * vertical != 0: periodic x, south face at T_hot, north at T_cold; 0: four
+ * walls, west face at T_hot, east at T_cold.  No temperature or moment field
+ * is written.  KB_F64 or KB_F32. */
+int kb_rayleigh_step_2d(void *f_out, const void *f_in, void *g_out, const void *g_in, int Nx, int Ny,
+                        double omega_f, double omega_T, double beta_g, double T_ref, double T_hot,
+                        double T_cold, int vertical, int dtype, void *stream);
+
 /* compute_temperature_2d!(Temp, g) -- src/kernels/thermal_2d.jl:113 */
 int kb_compute_temperature_2d(void *Temp, const void *g, int Nx, int Ny, int dtype, void *stream);
 
@@ -323,6 +333,21 @@ int kb_apply_zou_he_top_3d(void *f, double u_wall_x, int Nx, int Ny, int Nz, int
  *   -- src/kernels/boundary_3d.jl:232-288, 307-312 */
 int kb_apply_zou_he_pressure_3d(void *f, int Nx, int Ny, int Nz, int face, double rho_out,
                                 int dtype, void *stream);
+
+/* One step of run_cavity_3d (src/drivers/basic.jl:153-176) in one launch, same
+ * bits as stream_3d!, apply_zou_he_top_3d!, collide_3d! and, where rho/ux/uy/uz
+ * are given (all or none), compute_macroscopic_3d!. */
+int kb_cavity_step_3d(void *f_out, const void *f_in, void *rho, void *ux, void *uy, void *uz,
+                      const uint8_t *is_solid, int Nx, int Ny, int Nz, double omega, double u_lid,
+                      int dtype, void *stream);
+
+/* One step of run_natural_convection_3d (src/drivers/thermal.jl:455-537) in
+ * one launch, FP64 bits as the separate calls: stream f and g (six walls),
+ * west face at T_hot, east face at T_cold, temperature, moments, thermal BGK,
+ * Boussinesq BGK.  No temperature or moment field is written.  KB_F64 or KB_F32. */
+int kb_natconv_step_3d(void *f_out, const void *f_in, void *g_out, const void *g_in, int Nx, int Ny,
+                       int Nz, double omega_f, double omega_T, double beta_g, double T_ref,
+                       double T_hot, double T_cold, int dtype, void *stream);
 
 /* compute_macroscopic_3d!(rho, ux, uy, uz, f) -- src/kernels/macroscopic.jl:75 */
 int kb_compute_macroscopic_3d(void *rho, void *ux, void *uy, void *uz, const void *f, int Nx,

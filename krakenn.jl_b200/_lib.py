@@ -77,6 +77,9 @@ SIGNATURES: dict[str, list] = {
     "kb_fused_natconv_step": [_vp, _cvp, _vp, _cvp, _vp, _i, _i, _d, _d, _d, _d, _d, _d, _i, _vp],
     "kb_fused_natconv_vt_step": [_vp, _cvp, _vp, _cvp, _vp, _i, _i, _d, _d, _d, _d, _d, _d, _d,
                                  _d, _i, _vp],
+    "kb_rayleigh_step_2d": [_vp, _cvp, _vp, _cvp, _i, _i, _d, _d, _d, _d, _d, _d, _i, _i, _vp],
+    "kb_cavity_step_3d": [_vp, _cvp, _vp, _vp, _vp, _vp, _u8p, _i, _i, _i, _d, _d, _i, _vp],
+    "kb_natconv_step_3d": [_vp, _cvp, _vp, _cvp, _i, _i, _i, _d, _d, _d, _d, _d, _d, _i, _vp],
     "kb_compute_temperature_2d": [_vp, _cvp, _i, _i, _i, _vp],
     "kb_collide_thermal_2d": [_vp, _cvp, _cvp, _i, _i, _d, _i, _vp],
     "kb_collide_thermal_masked_2d": [_vp, _cvp, _cvp, _u8p, _i, _i, _d, _i, _vp],

@@ -638,21 +638,31 @@ __global__ void __launch_bounds__(BX) stream_periodic_k(T *__restrict__ fo, cons
 
 // stream_periodic_x_wall_y_2d_kernel!: src/kernels/stream_periodic_2d.jl:5-55
 template <typename T>
+__device__ __forceinline__ void pull_px_wy(const T *__restrict__ fi, const Grid2<T> &g, int i, int j,
+                                           T *p) {
+    const int Nx = g.Nx, Ny = g.Ny;
+    const size_t c = g.at(i, j), P = g.plane;
+    const int jm1 = j > 0 ? j - 1 : j, jp1 = j < Ny - 1 ? j + 1 : j;
+    const int iw = i > 0 ? i - 1 : Nx - 1, ie = i < Nx - 1 ? i + 1 : 0;
+    p[0] = fi[c];
+    p[1] = fi[g.at(iw, j) + 1 * P];
+    p[2] = j > 0 ? fi[g.at(i, jm1) + 2 * P] : fi[c + 4 * P];
+    p[3] = fi[g.at(ie, j) + 3 * P];
+    p[4] = j < Ny - 1 ? fi[g.at(i, jp1) + 4 * P] : fi[c + 2 * P];
+    p[5] = j > 0 ? fi[g.at(iw, jm1) + 5 * P] : fi[c + 7 * P];
+    p[6] = j > 0 ? fi[g.at(ie, jm1) + 6 * P] : fi[c + 8 * P];
+    p[7] = j < Ny - 1 ? fi[g.at(ie, jp1) + 7 * P] : fi[c + 5 * P];
+    p[8] = j < Ny - 1 ? fi[g.at(iw, jp1) + 8 * P] : fi[c + 6 * P];
+}
+
+template <typename T>
 __global__ void __launch_bounds__(BX) stream_px_wy_k(T *__restrict__ fo, const T *__restrict__ fi,
                                                       Grid2<T> g) {
     NODE2
-    const int Nx = g.Nx, Ny = g.Ny;
-    const int jm1 = j > 0 ? j - 1 : j, jp1 = j < Ny - 1 ? j + 1 : j;
-    const int iw = i > 0 ? i - 1 : Nx - 1, ie = i < Nx - 1 ? i + 1 : 0;
-    fo[c + 0 * P] = fi[c];
-    fo[c + 1 * P] = fi[g.at(iw, j) + 1 * P];
-    fo[c + 2 * P] = j > 0 ? fi[g.at(i, jm1) + 2 * P] : fi[c + 4 * P];
-    fo[c + 3 * P] = fi[g.at(ie, j) + 3 * P];
-    fo[c + 4 * P] = j < Ny - 1 ? fi[g.at(i, jp1) + 4 * P] : fi[c + 2 * P];
-    fo[c + 5 * P] = j > 0 ? fi[g.at(iw, jm1) + 5 * P] : fi[c + 7 * P];
-    fo[c + 6 * P] = j > 0 ? fi[g.at(ie, jm1) + 6 * P] : fi[c + 8 * P];
-    fo[c + 7 * P] = j < Ny - 1 ? fi[g.at(ie, jp1) + 7 * P] : fi[c + 5 * P];
-    fo[c + 8 * P] = j < Ny - 1 ? fi[g.at(iw, jp1) + 8 * P] : fi[c + 6 * P];
+    T p[9];
+    pull_px_wy(fi, g, i, j, p);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) fo[c + q * P] = p[q];
 }
 
 // One step of run_cavity_2d (src/drivers/basic.jl:121-136) in one launch.
@@ -941,6 +951,69 @@ __global__ void __launch_bounds__(BX) boussinesq_k(T *__restrict__ f, const T *_
     }
 #pragma unroll
     for (int q = 0; q < 9; ++q) f[c + q * P] = p[q];
+}
+
+// One step of run_rayleigh_benard_2d (src/drivers/thermal.jl:101-130) in one
+// launch: stream f and g (XPER: periodic x, walled y; else four walls), the
+// two fixed-temperature faces (XPER: south at T_lo, north at T_hi; else west
+// at T_lo, east at T_hi), temperature, moments (without the half force),
+// thermal BGK and Boussinesq BGK.  Temperature and moments stay in registers;
+// the driver reads them only after its last step.  Same expressions as
+// stream_k / stream_px_wy_k, fixed_temp_k, temperature_k, macroscopic_k,
+// collide_thermal_k and boussinesq_k, so FP64 keeps their bits.  36 values
+// per node instead of the 97 that the eight launches move, and one launch:
+// the driver's grids are small enough that launches set its speed.
+template <typename T, bool XPER>
+__global__ void __launch_bounds__(BX) rayleigh_step_k(T *__restrict__ fo, const T *__restrict__ fi,
+                                                       T *__restrict__ go, const T *__restrict__ gi,
+                                                       Grid2<T> g, T w_f, T w_T, T beta_g, T T_ref,
+                                                       T T_lo, T T_hi) {
+    NODE2
+    T p[9], h[9];
+    if (XPER) {
+        pull_px_wy(gi, g, i, j, h);
+        pull_px_wy(fi, g, i, j, p);
+    } else {
+        pull_bb(gi, g, i, j, h);
+        pull_bb(fi, g, i, j, p);
+    }
+    const T wa = T(2) * T(1.0 / 9.0), we = T(2) * T(1.0 / 36.0);
+    if (XPER) {
+        if (j == 0) {
+            h[2] = -h[2] + wa * T_lo;
+            h[5] = -h[5] + we * T_lo;
+            h[6] = -h[6] + we * T_lo;
+        }
+        if (j == g.Ny - 1) {
+            h[4] = -h[4] + wa * T_hi;
+            h[8] = -h[8] + we * T_hi;
+            h[7] = -h[7] + we * T_hi;
+        }
+    } else {
+        if (i == 0) {
+            h[1] = -h[1] + wa * T_lo;
+            h[5] = -h[5] + we * T_lo;
+            h[8] = -h[8] + we * T_lo;
+        }
+        if (i == g.Nx - 1) {
+            h[3] = -h[3] + wa * T_hi;
+            h[6] = -h[6] + we * T_hi;
+            h[7] = -h[7] + we * T_hi;
+        }
+    }
+    const T Tl = h[0] + h[1] + h[2] + h[3] + h[4] + h[5] + h[6] + h[7] + h[8];
+    T rho, a, b;
+    macro_node(p, rho, a, b);
+    collide_thermal(h, a, b, w_T);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) go[c + q * P] = h[q];
+    const T fx = T(0), fy = beta_g * (Tl - T_ref);
+    const T inv = T(1) / rho;
+    const T u = ((p[1] - p[3] + p[5] - p[6] - p[7] + p[8]) + fx / T(2)) * inv;
+    const T v = ((p[2] - p[4] + p[5] + p[6] - p[7] - p[8]) + fy / T(2)) * inv;
+    collide_guo(p, rho, u, v, fx, fy, w_f);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) fo[c + q * P] = p[q];
 }
 
 // compute_macroscopic_forced_2d_kernel! (src/kernels/macroscopic.jl:84-99):
@@ -1394,6 +1467,26 @@ int kb_cavity_movingwall_step_2d(void *f_out, const void *f_in, void *rho, void 
         (cavity_movingwall_k<T><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
             (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
             (T)omega, (T)u_lid)));
+}
+
+int kb_rayleigh_step_2d(void *f_out, const void *f_in, void *g_out, const void *g_in, int Nx, int Ny,
+                        double omega_f, double omega_T, double beta_g, double T_ref, double T_hot,
+                        double T_cold, int vertical, int dtype, void *stream) {
+    const char *what = "kb_rayleigh_step_2d";
+    KB_REQUIRE(f_out && f_in && g_out && g_in, "%s: null population pointer", what);
+    KB_REQUIRE(f_out != f_in && g_out != g_in && f_out != g_out && f_out != g_in && g_out != f_in,
+               "%s: the output buffers must differ from each other and from the inputs", what);
+    if (int e = check_dims(what, Nx, Ny)) return e;
+    cudaStream_t s = kb::as_stream(stream);
+    KB_DISPATCH_PLAIN(what, dtype,
+        if (vertical)
+            (rayleigh_step_k<T, true><<<nodes_grid(Nx, Ny), BX, 0, s>>>(
+                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, grid2<T>(Nx, Ny), (T)omega_f,
+                (T)omega_T, (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold));
+        else
+            (rayleigh_step_k<T, false><<<nodes_grid(Nx, Ny), BX, 0, s>>>(
+                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, grid2<T>(Nx, Ny), (T)omega_f,
+                (T)omega_T, (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold)));
 }
 
 int kb_fused_natconv_step(void *f_out, const void *f_in, void *g_out, const void *g_in,

@@ -503,6 +503,20 @@ __device__ __forceinline__ T cdot(int q, T x, T y, T z) {
     return r;
 }
 
+// Thermal BGK of one node at temperature Tm: the body of
+// collide_thermal_3d_kernel!.
+template <typename T>
+__device__ __forceinline__ void collide_thermal_node(T *p, T Tm, T a, T b, T d, T wT) {
+    const T t3 = T(3);
+    p[0] = p[0] - wT * (p[0] - T(1.0 / 3.0) * Tm);
+#pragma unroll
+    for (int q = 1; q < 19; ++q) {
+        const T w = q < 7 ? T(1.0 / 18.0) : T(1.0 / 36.0);
+        const T geq = w * Tm * (T(1) + t3 * cdot(q, a, b, d));
+        p[q] = p[q] - wT * (p[q] - geq);
+    }
+}
+
 // collide_thermal_3d_kernel!: src/kernels/thermal_3d.jl:12-104
 template <typename T>
 __global__ void __launch_bounds__(BX) collide_thermal_k(T *__restrict__ gg, const T *__restrict__ ux,
@@ -515,14 +529,9 @@ __global__ void __launch_bounds__(BX) collide_thermal_k(T *__restrict__ gg, cons
     T Tm = p[0];
 #pragma unroll
     for (int q = 1; q < 19; ++q) Tm = Tm + p[q];
-    const T a = ux[c], b = uy[c], d = uz[c], t3 = T(3);
-    gg[c] = p[0] - wT * (p[0] - T(1.0 / 3.0) * Tm);
+    collide_thermal_node(p, Tm, ux[c], uy[c], uz[c], wT);
 #pragma unroll
-    for (int q = 1; q < 19; ++q) {
-        const T w = q < 7 ? T(1.0 / 18.0) : T(1.0 / 36.0);
-        const T geq = w * Tm * (T(1) + t3 * cdot(q, a, b, d));
-        gg[c + q * P] = p[q] - wT * (p[q] - geq);
-    }
+    for (int q = 0; q < 19; ++q) gg[c + q * P] = p[q];
 }
 
 // compute_temperature_3d_kernel!: src/kernels/thermal_3d.jl:128-135
@@ -697,6 +706,125 @@ __global__ void __launch_bounds__(BX, 4) boussinesq2_k(float *__restrict__ f, co
     for (int q = 0; q < 19; ++q) *reinterpret_cast<float2 *>(f + c + q * P) = o[q].v;
 }
 
+// ---------------------------------------------------------- fused driver steps --
+// One step of run_cavity_3d (src/drivers/basic.jl:153-176) in one launch:
+// stream_3d!, apply_zou_he_top_3d! (face 5 of kFaces, u_n = 0, tangent x =
+// u_lid) on the top plane, collide_3d!, and compute_macroscopic_3d! of the
+// result where moments are asked for.  After the pull every stage touches
+// this node only, with the expressions of stream_k, zou_he_velocity_k,
+// collide_k and macroscopic_k, so the bits are theirs.  Memory bound: 38
+// values per node instead of the 99 that the four launches move.
+template <typename T>
+__device__ __forceinline__ void zou_he_top_node(T *p, T u_t1) {
+    const T u_n = T(0), u_t2 = T(0), sg = T(1);
+    T sum_par = T(0), sum_out = T(0);
+    const int par[9] = {0, 1, 2, 3, 4, 7, 8, 9, 10}, out[5] = {5, 11, 12, 15, 16};
+#pragma unroll
+    for (int n = 0; n < 9; ++n) sum_par += p[par[n]];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) sum_out += p[out[n]];
+    const T denom = T(1) + sg * u_n;
+    const T rw = (sum_par + T(2) * sum_out) / denom;
+    p[6] = p[5] - sg * T(1.0 / 3.0) * rw * u_n;
+    const T d1 = p[7], d2 = p[8], d3 = p[9], d4 = p[10];
+    const T t1 = (p[1] - p[2]) + (d1 - d2 + d3 - d4);
+    const T t2 = (p[3] - p[4]) + (d1 + d2 - d3 - d4);
+    const T s6 = sg * T(1.0 / 6.0);
+    p[13] = p[12] - T(0.5) * t1 + T(0.5) * rw * u_t1 - s6 * rw * u_n;
+    p[14] = p[11] + T(0.5) * t1 - T(0.5) * rw * u_t1 - s6 * rw * u_n;
+    p[17] = p[16] - T(0.5) * t2 + T(0.5) * rw * u_t2 - s6 * rw * u_n;
+    p[18] = p[15] + T(0.5) * t2 - T(0.5) * rw * u_t2 - s6 * rw * u_n;
+}
+
+template <typename T, typename I>
+__global__ void __launch_bounds__(BX) cavity_step_k(T *__restrict__ fo, const T *__restrict__ fi,
+                                                     T *__restrict__ rho, T *__restrict__ ux,
+                                                     T *__restrict__ uy, T *__restrict__ uz,
+                                                     const uint8_t *__restrict__ solid, Grid3 g,
+                                                     T omega, T u_lid) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y, k = blockIdx.z;
+    if (i >= g.Nx) return;
+    const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
+    const I P = (I)g.plane;
+    T p[19];
+    pull19_at(fi + c, P, pull_geometry<I>(g, i, j, k), p, Ident());
+    if (k == g.Nz - 1) zou_he_top_node(p, u_lid);
+    if (solid && solid[c]) {
+        swap_pairs(p);
+    } else {
+        T r, a, b, d, feq[19];
+        moments(p, r, a, b, d);
+        const T usq = a * a + b * b + d * d;
+        feq_all(r, a, b, d, usq, feq);
+#pragma unroll
+        for (int q = 0; q < 19; ++q) p[q] = p[q] - omega * (p[q] - feq[q]);
+    }
+    T *__restrict__ o0 = fo + c;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) o0[q * P] = p[q];
+    if (rho) {
+        T r, a, b, d;
+        moments(p, r, a, b, d);
+        rho[c] = r; ux[c] = a; uy[c] = b; uz[c] = d;
+    }
+}
+
+// One step of run_natural_convection_3d (src/drivers/thermal.jl:455-537) in
+// one launch: stream f and g, hot west / cold east anti-bounce-back faces,
+// temperature, moments (without the half force), thermal BGK, Boussinesq BGK
+// along y.  The temperature and the moments stay in registers; the driver
+// reads them only after its last step.  Same expressions as stream_k,
+// fixed_temp_k, temperature_k, macroscopic_k, collide_thermal_k and
+// boussinesq_k, so FP64 keeps their bits.  76 values per node instead of the
+// 199 of the eight launches.  g is collided and stored before f's collision
+// starts, so the 19 equilibria of f do not live beside both populations.
+template <typename T, typename I>
+__global__ void __launch_bounds__(BX, 3) natconv_step_k(T *__restrict__ fo, const T *__restrict__ fi,
+                                                      T *__restrict__ go, const T *__restrict__ gi,
+                                                      Grid3 g, T w_f, T w_T, T beta_g, T T_ref,
+                                                      T T_hot, T T_cold) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y, k = blockIdx.z;
+    if (i >= g.Nx) return;
+    const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
+    const I P = (I)g.plane;
+    const Pull3<I> s = pull_geometry<I>(g, i, j, k);
+    T p[19], h[19];
+    pull19_at(gi + c, P, s, h, Ident());
+    pull19_at(fi + c, P, s, p, Ident());
+    const T wa = T(2) * T(1.0 / 18.0), we = T(2) * T(1.0 / 36.0);
+    if (i == 0) {
+        h[1] = -h[1] + wa * T_hot;
+        h[7] = -h[7] + we * T_hot;
+        h[9] = -h[9] + we * T_hot;
+        h[11] = -h[11] + we * T_hot;
+        h[13] = -h[13] + we * T_hot;
+    }
+    if (i == g.Nx - 1) {
+        h[2] = -h[2] + wa * T_cold;
+        h[8] = -h[8] + we * T_cold;
+        h[10] = -h[10] + we * T_cold;
+        h[12] = -h[12] + we * T_cold;
+        h[14] = -h[14] + we * T_cold;
+    }
+    T Tm = h[0];
+#pragma unroll
+    for (int q = 1; q < 19; ++q) Tm = Tm + h[q];
+    {
+        T r, a, b, d;
+        moments(p, r, a, b, d);
+        collide_thermal_node(h, Tm, a, b, d, w_T);
+    }
+    T *__restrict__ g0 = go + c;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) g0[q * P] = h[q];
+    forced_bgk_node(p, w_f, T(0), beta_g * (Tm - T_ref), T(0));
+    T *__restrict__ o0 = fo + c;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) o0[q * P] = p[q];
+}
+
 }  // namespace d3
 }  // namespace kb
 
@@ -837,6 +965,49 @@ int kb_apply_zou_he_pressure_3d(void *f, int Nx, int Ny, int Nz, int face, doubl
     KB3_DISPATCH_PLAIN("kb_apply_zou_he_pressure_3d", dtype,
         (zou_he_pressure_k<T><<<grid, BX, 0, kb::as_stream(stream)>>>(
             (T *)f, grid3(Nx, Ny, Nz), F, fixed, N1, N2, (T)rho_out)));
+}
+
+int kb_cavity_step_3d(void *f_out, const void *f_in, void *rho, void *ux, void *uy, void *uz,
+                      const uint8_t *is_solid, int Nx, int Ny, int Nz, double omega, double u_lid,
+                      int dtype, void *stream) {
+    const char *what = "kb_cavity_step_3d";
+    KB_REQUIRE(f_out && f_in, "%s: null population pointer", what);
+    KB_REQUIRE(f_out != f_in, "%s: f_out and f_in must differ", what);
+    const int nm = (rho != nullptr) + (ux != nullptr) + (uy != nullptr) + (uz != nullptr);
+    KB_REQUIRE(nm == 0 || nm == 4, "%s: pass all four moment arrays or none", what);
+    if (int e = check_dims(what, Nx, Ny, Nz)) return e;
+    const Grid3 g = grid3(Nx, Ny, Nz);
+    cudaStream_t s = kb::as_stream(stream);
+    KB3_DISPATCH_PLAIN(what, dtype,
+        if (offsets_fit_int(g, 19))
+            (cavity_step_k<T, int><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+                (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
+                (T)u_lid));
+        else
+            (cavity_step_k<T, long long><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+                (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
+                (T)u_lid)));
+}
+
+int kb_natconv_step_3d(void *f_out, const void *f_in, void *g_out, const void *g_in, int Nx, int Ny,
+                       int Nz, double omega_f, double omega_T, double beta_g, double T_ref,
+                       double T_hot, double T_cold, int dtype, void *stream) {
+    const char *what = "kb_natconv_step_3d";
+    KB_REQUIRE(f_out && f_in && g_out && g_in, "%s: null population pointer", what);
+    KB_REQUIRE(f_out != f_in && g_out != g_in && f_out != g_out && f_out != g_in && g_out != f_in,
+               "%s: the output buffers must differ from each other and from the inputs", what);
+    if (int e = check_dims(what, Nx, Ny, Nz)) return e;
+    const Grid3 g = grid3(Nx, Ny, Nz);
+    cudaStream_t s = kb::as_stream(stream);
+    KB3_DISPATCH_PLAIN(what, dtype,
+        if (offsets_fit_int(g, 19))
+            (natconv_step_k<T, int><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
+                (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold));
+        else
+            (natconv_step_k<T, long long><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
+                (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold)));
 }
 
 int kb_compute_macroscopic_3d(void *rho, void *ux, void *uy, void *uz, const void *f, int Nx,

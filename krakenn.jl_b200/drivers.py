@@ -143,11 +143,12 @@ def run_cavity_3d(config: LBMConfig, backend="b200", T=torch.float64, on_step=No
     f_in, f_out = st["f_in"], st["f_out"]
     Nx, Ny, Nz = config.Nx, config.Ny, config.Nz
     w = omega(config)
+    fields = (st["rho"], st["ux"], st["uy"], st["uz"])
     for step in range(config.max_steps):
-        ops.stream_3d_(f_out, f_in, Nx, Ny, Nz)
-        ops.apply_zou_he_top_3d_(f_out, config.u_lid, Nx, Ny, Nz)
-        ops.collide_3d_(f_out, st["is_solid"], w)
-        ops.compute_macroscopic_3d_(st["rho"], st["ux"], st["uy"], st["uz"], f_out)
+        # every step overwrites the moments: they are written where something
+        # reads them (the hook, or the caller after the last step)
+        m = fields if on_step is not None or step == config.max_steps - 1 else (None,) * 4
+        ops.cavity_step_3d_(f_out, f_in, *m, None, Nx, Ny, Nz, w, config.u_lid)
         f_in, f_out = f_out, f_in
         if on_step is not None:
             on_step(step + 1, {"rho": st["rho"], "velocity": (st["ux"], st["uy"], st["uz"])})
@@ -411,9 +412,9 @@ def rayleigh_benard_parameters(Nx, Ny, Ra, Pr, T_hot=1.0, T_cold=0.0, nu=None, a
 def run_rayleigh_benard_2d(Nx=128, Ny=32, Ra=2000.0, Pr=1.0, T_hot=1.0, T_cold=0.0,
                            max_steps=20000, nu=None, alpha=None, orientation="vertical",
                            backend="b200", FT=torch.float64, graph=True):
-    """run_rayleigh_benard_2d -- src/drivers/thermal.jl:31-144: the unfused
-    DDF loop (stream f and g, fixed-temperature faces, T, moments, thermal
-    BGK, Boussinesq BGK) on the B200 kernels."""
+    """run_rayleigh_benard_2d -- src/drivers/thermal.jl:31-144: the DDF loop
+    (stream f and g, fixed-temperature faces, T, moments, thermal BGK,
+    Boussinesq BGK), one launch per step (kb_rayleigh_step_2d)."""
     _require_backend(backend)
     p = rayleigh_benard_parameters(Nx, Ny, Ra, Pr, T_hot, T_cold, nu, alpha, orientation)
     cfg = LBMConfig.d2q9(Nx, Ny, p["nu"], 0.0, max_steps)
@@ -422,23 +423,12 @@ def run_rayleigh_benard_2d(Nx=128, Ny=32, Ra=2000.0, Pr=1.0, T_hot=1.0, T_cold=0
     g0 = torch.from_numpy(rayleigh_benard_initial_g(Nx, Ny, T_hot, T_cold, orientation))
     g = [g0.to("cuda", FT), g0.to("cuda", FT)]
     Temp = torch.zeros((Ny, Nx), dtype=FT, device="cuda")
-    rho, ux, uy, solid = st["rho"], st["ux"], st["uy"], st["is_solid"]
-    stream = ops.stream_periodic_x_wall_y_2d_ if orientation == "vertical" else ops.stream_2d_
+    rho, ux, uy = st["rho"], st["ux"], st["uy"]
 
     def step(par):
-        fi, fo, gi, go = f[par], f[1 - par], g[par], g[1 - par]
-        stream(fo, fi, Nx, Ny)
-        stream(go, gi, Nx, Ny)
-        if orientation == "vertical":
-            ops.apply_fixed_temp_south_2d_(go, T_hot, Nx)
-            ops.apply_fixed_temp_north_2d_(go, T_cold, Nx, Ny)
-        else:
-            ops.apply_fixed_temp_west_2d_(go, T_hot, Ny)
-            ops.apply_fixed_temp_east_2d_(go, T_cold, Nx, Ny)
-        ops.compute_temperature_2d_(Temp, go)
-        ops.compute_macroscopic_2d_(rho, ux, uy, fo)
-        ops.collide_thermal_2d_(go, ux, uy, p["omega_T"])
-        ops.collide_boussinesq_2d_(fo, Temp, solid, p["omega_f"], p["beta_g"], p["T_ref"])
+        ops.rayleigh_step_2d_(f[1 - par], f[par], g[1 - par], g[par], Nx, Ny, p["omega_f"],
+                              p["omega_T"], p["beta_g"], p["T_ref"], T_hot, T_cold,
+                              orientation == "vertical")
 
     _step_loop(step, max_steps, graph)
     fin, gin = f[max_steps & 1], g[max_steps & 1]
@@ -482,7 +472,8 @@ def run_natural_convection_3d(N=32, Ra=1e3, Pr=0.71, T_hot=1.0, T_cold=0.0, max_
                               backend="b200", FT=torch.float64, graph=True):
     """run_natural_convection_3d -- src/drivers/thermal.jl:455-537: D3Q19
     flow and thermal DDF, hot west / cold east half-way walls, adiabatic
-    bounce-back elsewhere, Boussinesq force along y."""
+    bounce-back elsewhere, Boussinesq force along y; one launch per step
+    (kb_natconv_step_3d)."""
     _require_backend(backend)
     p = natconv_3d_parameters(N, Ra, Pr, T_hot, T_cold)
     cfg = LBMConfig.d3q19(N, N, N, p["nu"], 0.0, max_steps)
@@ -491,18 +482,11 @@ def run_natural_convection_3d(N=32, Ra=1e3, Pr=0.71, T_hot=1.0, T_cold=0.0, max_
     g0 = torch.from_numpy(np.ascontiguousarray(natconv_3d_initial_g(N, T_hot, T_cold)))
     g = [g0.to("cuda", FT), g0.to("cuda", FT)]
     Temp = torch.zeros((N, N, N), dtype=FT, device="cuda")
-    rho, ux, uy, uz, solid = st["rho"], st["ux"], st["uy"], st["uz"], st["is_solid"]
+    rho, ux, uy, uz = st["rho"], st["ux"], st["uy"], st["uz"]
 
     def step(par):
-        fi, fo, gi, go = f[par], f[1 - par], g[par], g[1 - par]
-        ops.stream_3d_(fo, fi, N, N, N)
-        ops.stream_3d_(go, gi, N, N, N)
-        ops.apply_fixed_temp_west_3d_(go, T_hot, N, N)
-        ops.apply_fixed_temp_east_3d_(go, T_cold, N, N, N)
-        ops.compute_temperature_3d_(Temp, go)
-        ops.compute_macroscopic_3d_(rho, ux, uy, uz, fo)
-        ops.collide_thermal_3d_(go, ux, uy, uz, p["omega_T"])
-        ops.collide_boussinesq_3d_(fo, Temp, solid, p["omega_f"], p["beta_g"], p["T_ref"])
+        ops.natconv_step_3d_(f[1 - par], f[par], g[1 - par], g[par], N, N, N, p["omega_f"],
+                             p["omega_T"], p["beta_g"], p["T_ref"], T_hot, T_cold)
 
     _step_loop(step, max_steps, graph)
     fin, gin = f[max_steps & 1], g[max_steps & 1]

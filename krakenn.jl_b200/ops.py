@@ -384,6 +384,22 @@ def cavity_mrt_step_2d_(f_out, f_in, rho, ux, uy, is_solid, Nx, Ny, nu, u_lid, s
          float(s_eps), float(s_q), float(u_lid), code, _stream())
 
 
+def rayleigh_step_2d_(f_out, f_in, g_out, g_in, Nx, Ny, omega_f, omega_T, beta_g, T_ref, T_hot,
+                      T_cold, vertical):
+    """One run_rayleigh_benard_2d step (src/drivers/thermal.jl:101-130) in one
+    launch.  vertical: periodic x, hot south and cold north walls; otherwise
+    four walls, hot west and cold east.  No field of T, rho or u is written."""
+    code = _plain(f_in)
+    for name, t in (("f_out", f_out), ("g_out", g_out), ("g_in", g_in)):
+        if t.dtype != f_in.dtype:
+            raise _arg_error(f"{name} must be a {f_in.dtype} tensor")
+    for t in (f_in, f_out, g_in, g_out):
+        _match2(t, Nx, Ny)
+    call("kb_rayleigh_step_2d", _t(f_out, "f_out"), _t(f_in, "f_in"), _t(g_out, "g_out"),
+         _t(g_in, "g_in"), Nx, Ny, float(omega_f), float(omega_T), float(beta_g), float(T_ref),
+         float(T_hot), float(T_cold), int(bool(vertical)), code, _stream())
+
+
 def _natconv_code(f_in, g_in, deviation, stochastic_rounding):
     """kb_dtype of a natural-convection step: the reference's FP64 / FP32, or
     (deviation) f - w_q and g - w_q T_ref in float32 / float16 / bfloat16."""
@@ -594,6 +610,34 @@ def compute_macroscopic_3d_(rho, ux, uy, uz, f):
     _ptrs_3d_fields(code, Nx, Ny, Nz, rho=rho, ux=ux, uy=uy, uz=uz)
     call("kb_compute_macroscopic_3d", _t(rho, "rho"), _t(ux, "ux"), _t(uy, "uy"), _t(uz, "uz"),
          _t(f, "f"), Nx, Ny, Nz, code, _stream())
+
+
+def cavity_step_3d_(f_out, f_in, rho, ux, uy, uz, is_solid, Nx, Ny, Nz, omega, u_lid):
+    """One run_cavity_3d step (src/drivers/basic.jl:153-176) in one launch;
+    moments may be None (then not written)."""
+    code = _plain(f_in)
+    if f_out.dtype != f_in.dtype:
+        raise _arg_error(f"f_out must be a {f_in.dtype} tensor")
+    _match3(f_in, Nx, Ny, Nz); _match3(f_out, Nx, Ny, Nz)
+    _ptrs_3d_fields(code, Nx, Ny, Nz, rho=rho, ux=ux, uy=uy, uz=uz)
+    call("kb_cavity_step_3d", _t(f_out, "f_out"), _t(f_in, "f_in"), _t(rho, "rho"), _t(ux, "ux"),
+         _t(uy, "uy"), _t(uz, "uz"), _mask(is_solid), Nx, Ny, Nz, float(omega), float(u_lid), code,
+         _stream())
+
+
+def natconv_step_3d_(f_out, f_in, g_out, g_in, Nx, Ny, Nz, omega_f, omega_T, beta_g, T_ref, T_hot,
+                     T_cold):
+    """One run_natural_convection_3d step (src/drivers/thermal.jl:455-537) in
+    one launch.  No field of T, rho or u is written."""
+    code = _plain(f_in)
+    for name, t in (("f_out", f_out), ("g_out", g_out), ("g_in", g_in)):
+        if t.dtype != f_in.dtype:
+            raise _arg_error(f"{name} must be a {f_in.dtype} tensor")
+    for t in (f_in, f_out, g_in, g_out):
+        _match3(t, Nx, Ny, Nz)
+    call("kb_natconv_step_3d", _t(f_out, "f_out"), _t(f_in, "f_in"), _t(g_out, "g_out"),
+         _t(g_in, "g_in"), Nx, Ny, Nz, float(omega_f), float(omega_T), float(beta_g), float(T_ref),
+         float(T_hot), float(T_cold), code, _stream())
 
 
 def collide_thermal_3d_(g, ux, uy, uz, omega_T):
