@@ -65,14 +65,23 @@ def _dev(device):
     return torch.device(device if device is not None else "cuda")
 
 
+def _weighted(W, field, shape, T, device):
+    """w_q * field at every node as a (Q, *shape) tensor of dtype T on the
+    device; `field` is a float64 host array that broadcasts to `shape`.  The
+    products are formed in float64 on the device and rounded once to T (the
+    values of the host expression), so only `field` crosses the bus."""
+    fd = torch.from_numpy(np.ascontiguousarray(field, dtype=np.float64)).to(device)
+    f = torch.empty((len(W),) + tuple(shape), dtype=T, device=device)
+    for q, w in enumerate(W):
+        f[q] = float(w) * fd
+    return f
+
+
 def initialize_2d(config: LBMConfig, T=torch.float64, device=None):
     """initialize_2d -- src/drivers/basic.jl:51-73 (f = w_q, rho = 1, u = 0)."""
     d = _dev(device)
     Nx, Ny = config.Nx, config.Ny
-    f_host = np.empty((9, Ny, Nx), dtype=np.float64)
-    for q in range(9):
-        f_host[q] = L.D2Q9_W[q]
-    f_in = torch.from_numpy(f_host).to(device=d, dtype=T)
+    f_in = _weighted(L.D2Q9_W, np.ones((1, 1)), (Ny, Nx), T, d)
     f_out = f_in.clone()
     return dict(f_in=f_in, f_out=f_out,
                 rho=torch.ones((Ny, Nx), dtype=T, device=d),
@@ -85,11 +94,8 @@ def initialize_3d(config: LBMConfig, T=torch.float64, device=None):
     """initialize_3d -- src/drivers/basic.jl:80-101"""
     d = _dev(device)
     Nx, Ny, Nz = config.Nx, config.Ny, config.Nz
-    f_host = np.empty((19, Nz, Ny, Nx), dtype=np.float64)
-    for q in range(19):
-        f_host[q] = L.D3Q19_W[q]
-    f_in = torch.from_numpy(f_host).to(device=d, dtype=T)
     shape = (Nz, Ny, Nx)
+    f_in = _weighted(L.D3Q19_W, np.ones((1, 1, 1)), shape, T, d)
     return dict(f_in=f_in, f_out=f_in.clone(),
                 rho=torch.ones(shape, dtype=T, device=d),
                 ux=torch.zeros(shape, dtype=T, device=d),
@@ -116,22 +122,31 @@ def run_cavity_2d(config: LBMConfig, backend="b200", T=torch.float64, fused=True
     st = state if state is not None else initialize_2d(config, T)
     f_in, f_out = st["f_in"], st["f_out"]
     rho, ux, uy, solid = st["rho"], st["ux"], st["uy"], st["is_solid"]
+    if state is None:
+        solid = None  # a fresh state has no solid node
     Nx, Ny = config.Nx, config.Ny
     w = omega(config)
-    for step in range(config.max_steps):
+    f = [f_in, f_out]
+
+    def step(par):
+        fi, fo = f[par], f[1 - par]
         if lid == "moving_wall":
-            ops.cavity_movingwall_step_2d_(f_out, f_in, rho, ux, uy, solid, Nx, Ny, w, config.u_lid)
+            ops.cavity_movingwall_step_2d_(fo, fi, rho, ux, uy, solid, Nx, Ny, w, config.u_lid)
         elif fused:
-            ops.cavity_step_2d_(f_out, f_in, rho, ux, uy, solid, Nx, Ny, w, config.u_lid)
+            ops.cavity_step_2d_(fo, fi, rho, ux, uy, solid, Nx, Ny, w, config.u_lid)
         else:
-            ops.stream_2d_(f_out, f_in, Nx, Ny)
-            ops.apply_zou_he_north_2d_(f_out, config.u_lid, Nx, Ny)
-            ops.collide_2d_(f_out, solid, w)
-            ops.compute_macroscopic_2d_(rho, ux, uy, f_out)
-        f_in, f_out = f_out, f_in
-        if on_step is not None:
-            on_step(step + 1, {"rho": rho, "velocity": (ux, uy)})
-    st["f_in"], st["f_out"] = f_in, f_out
+            ops.stream_2d_(fo, fi, Nx, Ny)
+            ops.apply_zou_he_north_2d_(fo, config.u_lid, Nx, Ny)
+            ops.collide_2d_(fo, solid, w)
+            ops.compute_macroscopic_2d_(rho, ux, uy, fo)
+
+    if on_step is None:
+        _step_loop(step, config.max_steps, True)
+    else:
+        for n in range(config.max_steps):
+            step(n & 1)
+            on_step(n + 1, {"rho": rho, "velocity": (ux, uy)})
+    st["f_in"], st["f_out"] = f[config.max_steps & 1], f[1 - (config.max_steps & 1)]
     return dict(rho=rho.cpu().numpy(), ux=ux.cpu().numpy(), uy=uy.cpu().numpy(), config=config,
                 state=st)
 
@@ -140,18 +155,24 @@ def run_cavity_3d(config: LBMConfig, backend="b200", T=torch.float64, on_step=No
     """run_cavity_3d -- src/drivers/basic.jl:153-176 (on_step as run_cavity_2d)"""
     _require_backend(backend)
     st = initialize_3d(config, T)
-    f_in, f_out = st["f_in"], st["f_out"]
+    f = [st["f_in"], st["f_out"]]
     Nx, Ny, Nz = config.Nx, config.Ny, config.Nz
     w = omega(config)
     fields = (st["rho"], st["ux"], st["uy"], st["uz"])
-    for step in range(config.max_steps):
-        # every step overwrites the moments: they are written where something
-        # reads them (the hook, or the caller after the last step)
-        m = fields if on_step is not None or step == config.max_steps - 1 else (None,) * 4
-        ops.cavity_step_3d_(f_out, f_in, *m, None, Nx, Ny, Nz, w, config.u_lid)
-        f_in, f_out = f_out, f_in
-        if on_step is not None:
-            on_step(step + 1, {"rho": st["rho"], "velocity": (st["ux"], st["uy"], st["uz"])})
+
+    def step(par, m=(None,) * 4):
+        ops.cavity_step_3d_(f[1 - par], f[par], *m, None, Nx, Ny, Nz, w, config.u_lid)
+
+    # every step overwrites the moments: they are written where something
+    # reads them (the hook, or the caller after the last step)
+    n = config.max_steps
+    if on_step is None and n > 0:
+        _step_loop(step, n - 1, True)
+        step((n - 1) & 1, fields)
+    elif on_step is not None:
+        for k in range(n):
+            step(k & 1, fields)
+            on_step(k + 1, {"rho": st["rho"], "velocity": (st["ux"], st["uy"], st["uz"])})
     return dict(rho=st["rho"].cpu().numpy(), ux=st["ux"].cpu().numpy(),
                 uy=st["uy"].cpu().numpy(), uz=st["uz"].cpu().numpy(), config=config)
 
@@ -220,10 +241,14 @@ def run_taylor_green_2d(N=64, nu=0.01, u0=0.01, max_steps=1000, backend="b200",
     f_out = f_in.clone()
     solid = torch.zeros((N, N), dtype=torch.bool, device="cuda")
     w = 1.0 / (3.0 * nu + 0.5)
-    for _ in range(max_steps):
-        ops.stream_fully_periodic_2d_(f_out, f_in, N, N)
-        ops.collide_2d_(f_out, solid, w)
-        f_in, f_out = f_out, f_in
+    f = [f_in, f_out]
+
+    def step(par):
+        ops.stream_fully_periodic_2d_(f[1 - par], f[par], N, N)
+        ops.collide_2d_(f[1 - par], solid, w)
+
+    _step_loop(step, max_steps, True)
+    f_in = f[max_steps & 1]
     rho = torch.empty((N, N), dtype=T, device="cuda")
     ux, uy = torch.empty_like(rho), torch.empty_like(rho)
     ops.compute_macroscopic_2d_(rho, ux, uy, f_in)
@@ -293,13 +318,18 @@ def natconv_parameters(N, Ra, Pr, T_hot=1.0, T_cold=0.0):
                 omega_T=1.0 / (3.0 * alpha + 0.5), T_ref=(T_hot + T_cold) / 2)
 
 
-def natconv_initial_g(N, T_hot=1.0, T_cold=0.0):
-    """g = w_q T_init with the linear profile + 1 % seed (thermal.jl:197-206)."""
+def _natconv_initial_T(N, T_hot, T_cold):
+    """Linear profile + 1 % seed of run_natural_convection_2d (thermal.jl:197-206)."""
     dT = T_hot - T_cold
     i = np.arange(1, N + 1, dtype=np.float64)[None, :]
     j = np.arange(1, N + 1, dtype=np.float64)[:, None]
     T0 = T_hot - dT * (i - 0.5) / N
-    T0 = T0 + (0.01 * dT) * np.sin(2 * math.pi * i / N) * np.sin(math.pi * j / N)
+    return T0 + (0.01 * dT) * np.sin(2 * math.pi * i / N) * np.sin(math.pi * j / N)
+
+
+def natconv_initial_g(N, T_hot=1.0, T_cold=0.0):
+    """g = w_q T_init with the linear profile + 1 % seed (thermal.jl:197-206)."""
+    T0 = _natconv_initial_T(N, T_hot, T_cold)
     return np.stack([L.D2Q9_W[q] * T0 for q in range(9)])
 
 
@@ -321,21 +351,23 @@ def run_natural_convection_2d(N=128, Ra=1e4, Pr=0.71, Rc=1.0, T_hot=1.0, T_cold=
     p = natconv_parameters(N, Ra, Pr, T_hot, T_cold)
     cfg = LBMConfig.d2q9(N, N, p["nu"], 0.0, max_steps)
     st = initialize_2d(cfg, FT)
-    f_in, f_out = st["f_in"], st["f_out"]
-    g_in = torch.from_numpy(natconv_initial_g(N, T_hot, T_cold)).to("cuda", FT)
-    g_out = g_in.clone()
+    f = [st["f_in"], st["f_out"]]
+    g_in = _weighted(L.D2Q9_W, _natconv_initial_T(N, T_hot, T_cold), (N, N), FT, "cuda")
+    g = [g_in, g_in.clone()]
     Temp = torch.zeros((N, N), dtype=FT, device="cuda")
     a_visc = -math.log(Rc)
-    for _ in range(max_steps):
+
+    def step(par):
+        fi, fo, gi, go = f[par], f[1 - par], g[par], g[1 - par]
         if Rc == 1.0:
-            ops.fused_natconv_step_(f_out, f_in, g_out, g_in, Temp, N, N, p["omega_f"],
-                                    p["omega_T"], p["beta_g"], p["T_ref"], T_hot, T_cold)
+            ops.fused_natconv_step_(fo, fi, go, gi, Temp, N, N, p["omega_f"], p["omega_T"],
+                                    p["beta_g"], p["T_ref"], T_hot, T_cold)
         else:
-            ops.fused_natconv_vt_step_(f_out, f_in, g_out, g_in, Temp, N, N, p["nu"], T_cold,
-                                       a_visc, p["omega_T"], p["beta_g"], p["T_ref"], T_hot,
-                                       T_cold)
-        f_in, f_out = f_out, f_in
-        g_in, g_out = g_out, g_in
+            ops.fused_natconv_vt_step_(fo, fi, go, gi, Temp, N, N, p["nu"], T_cold, a_visc,
+                                       p["omega_T"], p["beta_g"], p["T_ref"], T_hot, T_cold)
+
+    _step_loop(step, max_steps, True)
+    f_in, g_in = f[max_steps & 1], g[max_steps & 1]
     ops.compute_macroscopic_2d_(st["rho"], st["ux"], st["uy"], f_in)
     ops.compute_temperature_2d_(Temp, g_in)
     T_cpu = Temp.cpu().numpy()
@@ -346,33 +378,37 @@ def run_natural_convection_2d(N=128, Ra=1e4, Pr=0.71, Rc=1.0, T_hot=1.0, T_cold=
 
 # ------------------------------------------------ unfused thermal DDF drivers
 
+_CYCLE = 16  # steps per captured graph
+
+
 def _step_loop(step, max_steps: int, graph: bool):
     """Run `step(parity)` for parity = 0, 1, 0, ... max_steps times.  With
-    `graph`, one two-step cycle (which returns the ping-pong buffers to their
-    places) is captured once as a CUDA graph and replayed, so the short
-    boundary and collision launches of each step cost one graph launch."""
-    if not graph or max_steps < 4:
+    `graph`, _CYCLE steps (an even number, so the ping-pong buffers return to
+    their places) are captured once as a CUDA graph and replayed.  A host call
+    per step costs 10 to 13 us, a step of a 128^2 grid about 2 us; one replay
+    queues 16 steps in about 8 us, so the device sets the pace.  Longer cycles
+    gain nothing there and delay the first step of a large grid by their
+    capture (10 us per captured step)."""
+    if not graph or max_steps < 2 * _CYCLE:
         for s in range(max_steps):
             step(s & 1)
         return
     from .batch import Graph
     g = Graph()
     with g:
-        step(0)
-        step(1)
+        for s in range(_CYCLE):
+            step(s & 1)
     try:
-        for _ in range(max_steps // 2):
+        for _ in range(max_steps // _CYCLE):
             g.launch()
-        if max_steps & 1:
-            step(0)
+        for s in range(max_steps % _CYCLE):
+            step(s & 1)
     finally:
         g.close()
 
 
-def rayleigh_benard_initial_g(Nx, Ny, T_hot=1.0, T_cold=0.0, orientation="vertical"):
-    """Thermal populations g = w_q T_init of run_rayleigh_benard_2d
-    (src/drivers/thermal.jl:79-98): the half-way conduction profile across
-    the heated gap, plus the sin-sin seed for the vertical orientation."""
+def _rayleigh_benard_initial_T(Nx, Ny, T_hot, T_cold, orientation):
+    """T_init of run_rayleigh_benard_2d (src/drivers/thermal.jl:79-98)."""
     dT = T_hot - T_cold
     i = np.arange(1, Nx + 1, dtype=np.float64)[None, :]
     j = np.arange(1, Ny + 1, dtype=np.float64)[:, None]
@@ -380,9 +416,15 @@ def rayleigh_benard_initial_g(Nx, Ny, T_hot=1.0, T_cold=0.0, orientation="vertic
         # the seed is separable: libm sin per row / column value
         si = np.array([math.sin(2 * math.pi * a / Nx) for a in range(1, Nx + 1)])[None, :]
         sj = np.array([math.sin(math.pi * b / Ny) for b in range(1, Ny + 1)])[:, None]
-        T0 = (T_hot - dT * (j - 0.5) / Ny) + ((0.01 * dT) * si) * sj
-    else:
-        T0 = np.broadcast_to(T_hot - dT * (i - 0.5) / Nx, (Ny, Nx))
+        return (T_hot - dT * (j - 0.5) / Ny) + ((0.01 * dT) * si) * sj
+    return np.broadcast_to(T_hot - dT * (i - 0.5) / Nx, (Ny, Nx))
+
+
+def rayleigh_benard_initial_g(Nx, Ny, T_hot=1.0, T_cold=0.0, orientation="vertical"):
+    """Thermal populations g = w_q T_init of run_rayleigh_benard_2d
+    (src/drivers/thermal.jl:79-98): the half-way conduction profile across
+    the heated gap, plus the sin-sin seed for the vertical orientation."""
+    T0 = _rayleigh_benard_initial_T(Nx, Ny, T_hot, T_cold, orientation)
     return np.stack([L.D2Q9_W[q] * T0 for q in range(9)])
 
 
@@ -420,8 +462,9 @@ def run_rayleigh_benard_2d(Nx=128, Ny=32, Ra=2000.0, Pr=1.0, T_hot=1.0, T_cold=0
     cfg = LBMConfig.d2q9(Nx, Ny, p["nu"], 0.0, max_steps)
     st = initialize_2d(cfg, FT)
     f = [st["f_in"], st["f_out"]]
-    g0 = torch.from_numpy(rayleigh_benard_initial_g(Nx, Ny, T_hot, T_cold, orientation))
-    g = [g0.to("cuda", FT), g0.to("cuda", FT)]
+    g0 = _weighted(L.D2Q9_W, _rayleigh_benard_initial_T(Nx, Ny, T_hot, T_cold, orientation),
+                   (Ny, Nx), FT, "cuda")
+    g = [g0, g0.clone()]
     Temp = torch.zeros((Ny, Nx), dtype=FT, device="cuda")
     rho, ux, uy = st["rho"], st["ux"], st["uy"]
 
@@ -446,6 +489,12 @@ def natconv_3d_initial_g(N, T_hot=1.0, T_cold=0.0):
     i = np.arange(1, N + 1, dtype=np.float64)
     T0 = np.broadcast_to(T_hot - dT * (i - 0.5) / N, (N, N, N))
     return np.stack([L.D3Q19_W[q] * T0 for q in range(19)])
+
+
+def _natconv_3d_initial_T(N, T_hot, T_cold):
+    """The x profile of natconv_3d_initial_g, broadcast along y and z."""
+    i = np.arange(1, N + 1, dtype=np.float64)
+    return (T_hot - (T_hot - T_cold) * (i - 0.5) / N)[None, None, :]
 
 
 def natconv_3d_parameters(N, Ra, Pr, T_hot=1.0, T_cold=0.0):
@@ -479,8 +528,8 @@ def run_natural_convection_3d(N=32, Ra=1e3, Pr=0.71, T_hot=1.0, T_cold=0.0, max_
     cfg = LBMConfig.d3q19(N, N, N, p["nu"], 0.0, max_steps)
     st = initialize_3d(cfg, FT)
     f = [st["f_in"], st["f_out"]]
-    g0 = torch.from_numpy(np.ascontiguousarray(natconv_3d_initial_g(N, T_hot, T_cold)))
-    g = [g0.to("cuda", FT), g0.to("cuda", FT)]
+    g0 = _weighted(L.D3Q19_W, _natconv_3d_initial_T(N, T_hot, T_cold), (N, N, N), FT, "cuda")
+    g = [g0, g0.clone()]
     Temp = torch.zeros((N, N, N), dtype=FT, device="cuda")
     rho, ux, uy, uz = st["rho"], st["ux"], st["uy"], st["uz"]
 
