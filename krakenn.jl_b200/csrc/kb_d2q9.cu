@@ -5,9 +5,10 @@
 // reference's CPU Float64 path bit for bit (and a float run its Float32
 // path).  Each kernel names the reference kernel it restates.
 //
-// Thread mapping: one thread per node, blockDim.x along x (the unit-stride
-// axis of every population plane), so each population load/store of a warp
-// is one contiguous run of 32 elements (shifted by one for the x-pulls).
+// Thread mapping: one thread per node, numbered along x (the unit-stride axis
+// of every population plane) and, where rows do not fill the blocks, on
+// through the rows (node_ij), so each population load/store of a warp is one
+// contiguous run of 32 elements (shifted by one for the x-pulls).
 #include "kb_common.cuh"
 
 namespace kb {
@@ -30,6 +31,7 @@ template <typename T>
 struct Grid2 {
     int Nx, Ny;
     size_t plane;  // Nx*Ny
+    unsigned magic;  // thread numbering (node_ij)
     __device__ __forceinline__ size_t at(int i, int j) const { return (size_t)i + (size_t)Nx * j; }
 };
 
@@ -102,9 +104,8 @@ __device__ __forceinline__ void bgk(T *p, T omega, T &rho, T &ux, T &uy) {
 }
 
 #define NODE2                                              \
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;   \
-    const int j = blockIdx.y;                              \
-    if (i >= g.Nx) return;                                 \
+    int i, j;                                              \
+    if (!node_ij(g.Nx, g.Ny, g.magic, i, j)) return;       \
     const size_t c = g.at(i, j);                           \
     const size_t P = g.plane;
 
@@ -1119,10 +1120,15 @@ template <typename T>
 Grid2<T> grid2(int Nx, int Ny) {
     Grid2<T> g;
     g.Nx = Nx; g.Ny = Ny; g.plane = (size_t)Nx * (size_t)Ny;
+    g.magic = kb::node_magic(Nx, Ny);
     return g;
 }
 
-inline dim3 nodes_grid(int Nx, int Ny) { return dim3((Nx + BX - 1) / BX, Ny); }
+static_assert(BX == kb::NODE_BX, "one-node kernels number nodes in blocks of NODE_BX");
+inline dim3 nodes_grid(int Nx, int Ny) {
+    const unsigned m = kb::node_magic(Nx, Ny);
+    return dim3(kb::node_blocks(Nx, Ny, m), m ? 1 : Ny);
+}
 inline unsigned line_grid(int n) { return (unsigned)((n + BX - 1) / BX); }
 
 // Forced BGK (KIND 0 Boussinesq, 1 constant Guo force, 2 per-node Guo force):

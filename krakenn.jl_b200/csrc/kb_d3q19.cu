@@ -64,10 +64,13 @@ struct Ident {
     template <typename V> __device__ __forceinline__ V operator()(V v) const { return v; }
 };
 
+#define NODE3_IJK                                                 \
+    int i, j;                                                     \
+    const int k = blockIdx.z;                                     \
+    if (!node_ij(g.Nx, g.Ny, g.magic, i, j)) return;
+
 #define NODE3                                                     \
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;          \
-    const int j = blockIdx.y, k = blockIdx.z;                     \
-    if (i >= g.Nx) return;                                        \
+    NODE3_IJK                                                     \
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k); \
     const size_t P = g.plane;
 
@@ -152,9 +155,7 @@ __global__ void __launch_bounds__(BX) fused_trt_k(T *__restrict__ fo, const T *_
                                                    T *__restrict__ uy, T *__restrict__ uz,
                                                    const uint8_t *__restrict__ solid, Grid3 g, T sp,
                                                    T sm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= g.Nx) return;
+    NODE3_IJK
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     T *__restrict__ o0 = fo + c;
@@ -197,9 +198,7 @@ __global__ void __launch_bounds__(BX) fused_trt_libb_k(T *__restrict__ fo, const
                                                         const T *__restrict__ wy,
                                                         const T *__restrict__ wz, Grid3 g, T sp,
                                                         T sm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= g.Nx) return;
+    NODE3_IJK
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     T *__restrict__ o0 = fo + c;
@@ -280,9 +279,7 @@ __global__ void __launch_bounds__(BX) fused_trt_links_k(T *__restrict__ fo, cons
                                                          T *__restrict__ rho, T *__restrict__ ux,
                                                          T *__restrict__ uy, T *__restrict__ uz,
                                                          LinkTable3 L, Grid3 g, T sp, T sm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= g.Nx) return;
+    NODE3_IJK
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const uint8_t cl = L.cls[c];
     if (SKIP_CUT) {
@@ -642,9 +639,7 @@ __global__ void __launch_bounds__(BX, sizeof(T) == 8 ? 4 : 1) boussinesq_k(T *__
                                                     T beta_g, T T_ref, const T *__restrict__ Fxf,
                                                     const T *__restrict__ Fyf,
                                                     const T *__restrict__ Fzf, T Fx, T Fy, T Fz) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= g.Nx) return;
+    NODE3_IJK
     const I c = (I)i + (I)g.Nx * ((I)j + (I)g.Ny * (I)k);
     const I P = (I)g.plane;
     T p[19];
@@ -742,9 +737,7 @@ __global__ void __launch_bounds__(BX) cavity_step_k(T *__restrict__ fo, const T 
                                                      T *__restrict__ uy, T *__restrict__ uz,
                                                      const uint8_t *__restrict__ solid, Grid3 g,
                                                      T omega, T u_lid) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= g.Nx) return;
+    NODE3_IJK
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     T p[19];
@@ -784,9 +777,7 @@ __global__ void __launch_bounds__(BX, 3) natconv_step_k(T *__restrict__ fo, cons
                                                       T *__restrict__ go, const T *__restrict__ gi,
                                                       Grid3 g, T w_f, T w_T, T beta_g, T T_ref,
                                                       T T_hot, T T_cold) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= g.Nx) return;
+    NODE3_IJK
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     const Pull3<I> s = pull_geometry<I>(g, i, j, k);
@@ -837,6 +828,7 @@ Grid3 grid3(int Nx, int Ny, int Nz, int per = 0) {
     Grid3 g;
     g.Nx = Nx; g.Ny = Ny; g.Nz = Nz; g.per = per;
     g.plane = (size_t)Nx * (size_t)Ny * (size_t)Nz;
+    g.magic = kb::node_magic(Nx, Ny);
     return g;
 }
 
@@ -882,7 +874,7 @@ template <typename T>
 void launch_trt_libb_3d(void *f_out, const void *f_in, void *rho, void *ux, void *uy, void *uz,
                         const uint8_t *solid, const void *qw, const void *wx, const void *wy,
                         const void *wz, const Grid3 &g, double sp, double sm, cudaStream_t s) {
-    const dim3 grid = nodes_grid(g.Nx, g.Ny, g.Nz);
+    const dim3 grid = node_grid(g);
     if (offsets_fit_int(g, 19))
         fused_trt_libb_k<T, int><<<grid, BX, 0, s>>>(
             (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, solid, (const T *)qw,
@@ -918,7 +910,7 @@ int kb_stream_3d(void *f_out, const void *f_in, int Nx, int Ny, int Nz, int dtyp
     KB_REQUIRE(f_out != f_in, "kb_stream_3d: f_out and f_in must differ");
     if (int e = check_dims("kb_stream_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_stream_3d", dtype,
-        (stream_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (stream_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)f_out, (const T *)f_in, grid3(Nx, Ny, Nz))));
 }
 
@@ -927,7 +919,7 @@ int kb_collide_3d(void *f, const uint8_t *is_solid, int Nx, int Ny, int Nz, doub
     KB_REQUIRE(f, "kb_collide_3d: null population pointer");
     if (int e = check_dims("kb_collide_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_collide_3d", dtype,
-        (collide_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (collide_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)f, is_solid, grid3(Nx, Ny, Nz), (T)omega)));
 }
 
@@ -980,11 +972,11 @@ int kb_cavity_step_3d(void *f_out, const void *f_in, void *rho, void *ux, void *
     cudaStream_t s = kb::as_stream(stream);
     KB3_DISPATCH_PLAIN(what, dtype,
         if (offsets_fit_int(g, 19))
-            (cavity_step_k<T, int><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+            (cavity_step_k<T, int><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
                 (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
                 (T)u_lid));
         else
-            (cavity_step_k<T, long long><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+            (cavity_step_k<T, long long><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
                 (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
                 (T)u_lid)));
 }
@@ -1001,11 +993,11 @@ int kb_natconv_step_3d(void *f_out, const void *f_in, void *g_out, const void *g
     cudaStream_t s = kb::as_stream(stream);
     KB3_DISPATCH_PLAIN(what, dtype,
         if (offsets_fit_int(g, 19))
-            (natconv_step_k<T, int><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+            (natconv_step_k<T, int><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
                 (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
                 (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold));
         else
-            (natconv_step_k<T, long long><<<nodes_grid(Nx, Ny, Nz), BX, 0, s>>>(
+            (natconv_step_k<T, long long><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
                 (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
                 (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold)));
 }
@@ -1015,7 +1007,7 @@ int kb_compute_macroscopic_3d(void *rho, void *ux, void *uy, void *uz, const voi
     KB_REQUIRE(rho && ux && uy && uz && f, "kb_compute_macroscopic_3d: null pointer");
     if (int e = check_dims("kb_compute_macroscopic_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_compute_macroscopic_3d", dtype,
-        (macroscopic_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (macroscopic_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)rho, (T *)ux, (T *)uy, (T *)uz, (const T *)f, grid3(Nx, Ny, Nz))));
 }
 
@@ -1035,7 +1027,7 @@ int trt3d_step(const char *what, void *f_out, const void *f_in, void *rho, void 
     if (int e = kb_trt_rates(nu, Lambda, &sp, &sm)) return e;
     cudaStream_t s = kb::as_stream(stream);
     const bool i32 = offsets_fit_int(g, 19);
-    const dim3 grid = nodes_grid(g.Nx, g.Ny, g.Nz);
+    const dim3 grid = node_grid(g);
     if (dtype == KB_F64) {
         if (i32)
             fused_trt_k<double, int><<<grid, BX, 0, s>>>(
@@ -1141,7 +1133,7 @@ int kb_stream_periodic_xz_movingwall_y_3d(void *f_out, const void *f_in, double 
     KB_REQUIRE(f_out != f_in, "kb_stream_periodic_xz_movingwall_y_3d: f_out and f_in must differ");
     if (int e = check_dims("kb_stream_periodic_xz_movingwall_y_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_stream_periodic_xz_movingwall_y_3d", dtype,
-        (movingwall_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (movingwall_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)f_out, (const T *)f_in, grid3(Nx, Ny, Nz), (T)Ub, (T)Ut, (T)rho_w)));
 }
 
@@ -1150,7 +1142,7 @@ int kb_collide_thermal_3d(void *g, const void *ux, const void *uy, const void *u
     KB_REQUIRE(g && ux && uy && uz, "kb_collide_thermal_3d: null pointer");
     if (int e = check_dims("kb_collide_thermal_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_collide_thermal_3d", dtype,
-        (collide_thermal_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (collide_thermal_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)g, (const T *)ux, (const T *)uy, (const T *)uz, grid3(Nx, Ny, Nz), (T)omega_T)));
 }
 
@@ -1159,7 +1151,7 @@ int kb_compute_temperature_3d(void *Temp, const void *g, int Nx, int Ny, int Nz,
     KB_REQUIRE(Temp && g, "kb_compute_temperature_3d: null pointer");
     if (int e = check_dims("kb_compute_temperature_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_compute_temperature_3d", dtype,
-        (temperature_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (temperature_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)Temp, (const T *)g, grid3(Nx, Ny, Nz))));
 }
 
@@ -1188,7 +1180,7 @@ void launch_boussinesq_3d(T *f, const T *Temp, const uint8_t *solid, const Grid3
             return;
         }
     }
-    const dim3 grid = nodes_grid(g.Nx, g.Ny, g.Nz);
+    const dim3 grid = node_grid(g);
     if (i32)
         boussinesq_k<T, MODE, int><<<grid, BX, 0, s>>>(f, Temp, solid, g, w, beta_g, T_ref, Fxf, Fyf,
                                                        Fzf, Fx, Fy, Fz);
@@ -1406,7 +1398,7 @@ int build_links(kb_libb_links *L, const uint8_t *solid, const T *qw, const T *wx
 template <typename T, typename I>
 int launch_links_3d_i(T *fo, const T *fi, T *rho, T *ux, T *uy, T *uz,
                        const kb::d3::LinkTable3 &L, const Grid3 &g, T sp, T sm, cudaStream_t s) {
-    const dim3 grid = nodes_grid(g.Nx, g.Ny, g.Nz);
+    const dim3 grid = node_grid(g);
     kb::d3::SideStream *ss = L.n_rec > 0 ? kb::d3::side_stream() : nullptr;
     if (!ss) {  // no cut nodes, or no side stream: one kernel for every node
         fused_trt_links_k<T, I, false><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
@@ -1527,7 +1519,7 @@ int kb_compute_macroscopic_forced_3d(void *rho, void *ux, void *uy, void *uz, co
     KB_REQUIRE(rho && ux && uy && uz && f, "kb_compute_macroscopic_forced_3d: null pointer");
     if (int e = check_dims("kb_compute_macroscopic_forced_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_compute_macroscopic_forced_3d", dtype,
-        (macroscopic_forced_k<T, false><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (macroscopic_forced_k<T, false><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)rho, (T *)ux, (T *)uy, (T *)uz, (const T *)f, grid3(Nx, Ny, Nz), (T)Fx, (T)Fy,
             (T)Fz, nullptr, nullptr, nullptr)));
 }
@@ -1540,7 +1532,7 @@ int kb_compute_macroscopic_forced_field_3d(void *rho, void *ux, void *uy, void *
                "kb_compute_macroscopic_forced_field_3d: null pointer");
     if (int e = check_dims("kb_compute_macroscopic_forced_field_3d", Nx, Ny, Nz)) return e;
     KB3_DISPATCH_PLAIN("kb_compute_macroscopic_forced_field_3d", dtype,
-        (macroscopic_forced_k<T, true><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (macroscopic_forced_k<T, true><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)rho, (T *)ux, (T *)uy, (T *)uz, (const T *)f, grid3(Nx, Ny, Nz), T(0), T(0),
             T(0), (const T *)Fx_field, (const T *)Fy_field, (const T *)Fz_field)));
 }
@@ -1552,7 +1544,7 @@ int kb_stream_periodic_xz_wall_y_3d(void *f_out, const void *f_in, int Nx, int N
     if (int e = check_dims("kb_stream_periodic_xz_wall_y_3d", Nx, Ny, Nz)) return e;
     // the pull of stream_3d with x and z wrapped (periodic mask x | z)
     KB3_DISPATCH_PLAIN("kb_stream_periodic_xz_wall_y_3d", dtype,
-        (stream_k<T><<<nodes_grid(Nx, Ny, Nz), BX, 0, kb::as_stream(stream)>>>(
+        (stream_k<T><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, kb::as_stream(stream)>>>(
             (T *)f_out, (const T *)f_in, grid3(Nx, Ny, Nz, 5))));
 }
 

@@ -17,6 +17,7 @@ struct Grid3 {
     size_t plane;  // population stride in nodes: Nx*Ny*Nz, or more for a z-range
     int per;       // bit 0 x, bit 1 y, bit 2 z periodic; bit 3 z halo (below)
     int zoff = 0;  // z-range: plane of the allocation that k = 0 is (staged copies)
+    unsigned magic = 0;  // thread numbering of the one-node kernels (node_ij)
 };
 // z halo (per bit 3): the grid is a range of z-planes inside a larger
 // allocation whose planes k = -1 and k = Nz exist; z-pulls read them as they
@@ -98,6 +99,12 @@ __device__ __forceinline__ void pull19(const R *__restrict__ f, size_t P, size_t
 inline bool offsets_fit_int(const Grid3 &g, int Q) {
     return (double)g.plane * (double)(Q + 1) < 2147483647.0;
 }
+
+// Launch grid of the one-node kernels on grid g (NODE3), BX threads a block.
+inline dim3 node_grid(const Grid3 &g) {
+    return dim3(node_blocks(g.Nx, g.Ny, g.magic), g.magic ? 1 : g.Ny, g.Nz);
+}
+static_assert(BX == NODE_BX, "one-node kernels number nodes in blocks of NODE_BX");
 
 inline dim3 nodes_grid(int Nx, int Ny, int Nz) { return dim3((Nx + BX - 1) / BX, Ny, Nz); }
 
