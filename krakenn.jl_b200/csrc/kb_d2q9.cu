@@ -320,6 +320,26 @@ __global__ void __launch_bounds__(BX) fused_bgk_k(T *__restrict__ fo, const T *_
     rho[c] = r; ux[c] = a; uy[c] = b;
 }
 
+// TRT update of one fluid node in place (fused_trt_2d.jl:29-101), with its moments.
+template <typename T>
+__device__ __forceinline__ void trt_node(T *p, T sp, T sm, T &r, T &a_, T &b_) {
+    T feq[9];
+    moments(p, r, a_, b_);
+    const T usq = a_ * a_ + b_ * b_;
+    feq_all(r, a_, b_, usq, feq);
+    const T a = (sp + sm) * T(0.5), b = (sp - sm) * T(0.5);
+    const T p1 = p[1], p2 = p[2], p5 = p[5], p6 = p[6];
+    p[0] = p[0] - sp * (p[0] - feq[0]);
+    p[1] = p1 - a * (p1 - feq[1]) - b * (p[3] - feq[3]);
+    p[3] = p[3] - a * (p[3] - feq[3]) - b * (p1 - feq[1]);
+    p[2] = p2 - a * (p2 - feq[2]) - b * (p[4] - feq[4]);
+    p[4] = p[4] - a * (p[4] - feq[4]) - b * (p2 - feq[2]);
+    p[5] = p5 - a * (p5 - feq[5]) - b * (p[7] - feq[7]);
+    p[7] = p[7] - a * (p[7] - feq[7]) - b * (p5 - feq[5]);
+    p[6] = p6 - a * (p6 - feq[6]) - b * (p[8] - feq[8]);
+    p[8] = p[8] - a * (p[8] - feq[8]) - b * (p6 - feq[6]);
+}
+
 // fused_trt_step_kernel!: src/kernels/fused_trt_2d.jl:29-101
 template <typename T>
 __global__ void __launch_bounds__(BX) fused_trt_k(T *__restrict__ fo, const T *__restrict__ fi,
@@ -338,20 +358,9 @@ __global__ void __launch_bounds__(BX) fused_trt_k(T *__restrict__ fo, const T *_
         rho[c] = T(1); ux[c] = T(0); uy[c] = T(0);
         return;
     }
-    T feq[9];
-    moments(p, r, a_, b_);
-    T usq = a_ * a_ + b_ * b_;
-    feq_all(r, a_, b_, usq, feq);
-    const T a = (sp + sm) * T(0.5), b = (sp - sm) * T(0.5);
-    fo[c + 0 * P] = p[0] - sp * (p[0] - feq[0]);
-    fo[c + 1 * P] = p[1] - a * (p[1] - feq[1]) - b * (p[3] - feq[3]);
-    fo[c + 3 * P] = p[3] - a * (p[3] - feq[3]) - b * (p[1] - feq[1]);
-    fo[c + 2 * P] = p[2] - a * (p[2] - feq[2]) - b * (p[4] - feq[4]);
-    fo[c + 4 * P] = p[4] - a * (p[4] - feq[4]) - b * (p[2] - feq[2]);
-    fo[c + 5 * P] = p[5] - a * (p[5] - feq[5]) - b * (p[7] - feq[7]);
-    fo[c + 7 * P] = p[7] - a * (p[7] - feq[7]) - b * (p[5] - feq[5]);
-    fo[c + 6 * P] = p[6] - a * (p[6] - feq[6]) - b * (p[8] - feq[8]);
-    fo[c + 8 * P] = p[8] - a * (p[8] - feq[8]) - b * (p[6] - feq[6]);
+    trt_node(p, sp, sm, r, a_, b_);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) fo[c + q * P] = p[q];
     rho[c] = r; ux[c] = a_; uy[c] = b_;
 }
 
@@ -819,6 +828,124 @@ __global__ void __launch_bounds__(BX) natconv_k(T *__restrict__ fo, const T *__r
     for (int q = 0; q < 9; ++q) fo[c + q * P] = fp[q];
 }
 
+// Pull of the adjacent nodes (i, j), (i + 1, j), i even, as two lanes: each
+// population the value pull_bb gives.  Rows are even and the planes 8-byte
+// aligned, so an unshifted population is one 8-byte load.
+template <typename I>
+__device__ __forceinline__ void pull_bb_pair(const float *__restrict__ f, int Nx, int Ny, I P, I c, int i,
+                                             int j, Lanes2 *p) {
+    const bool w = i > 0, e = i + 1 < Nx - 1, s = j > 0, n = j < Ny - 1;
+    const I N = (I)Nx;
+    const auto ld2 = [&](I o) { return *reinterpret_cast<const float2 *>(f + o); };
+    p[0].v = ld2(c);
+    p[2].v = ld2(s ? c - N + 2 * P : c + 4 * P);
+    p[4].v = ld2(n ? c + N + 4 * P : c + 2 * P);
+    p[1].v = make_float2(f[w ? c - 1 + P : c + 3 * P], f[c + P]);
+    p[3].v = make_float2(f[c + 1 + 3 * P], f[e ? c + 2 + 3 * P : c + 1 + P]);
+    p[5].v = make_float2(f[(w && s) ? c - 1 - N + 5 * P : c + 7 * P], f[s ? c - N + 5 * P : c + 1 + 7 * P]);
+    p[6].v = make_float2(f[s ? c + 1 - N + 6 * P : c + 8 * P],
+                         f[(e && s) ? c + 2 - N + 6 * P : c + 1 + 8 * P]);
+    p[7].v = make_float2(f[n ? c + 1 + N + 7 * P : c + 5 * P],
+                         f[(e && n) ? c + 2 + N + 7 * P : c + 1 + 5 * P]);
+    p[8].v = make_float2(f[(w && n) ? c - 1 + N + 8 * P : c + 6 * P], f[n ? c + N + 8 * P : c + 1 + 6 * P]);
+}
+
+// fused_bgk_k (TRT = false) and fused_trt_k (TRT = true) in FP32 for even Nx
+// and 8-byte aligned arrays: two adjacent nodes per thread, each with the
+// one-node kernel's scalar arithmetic, so the bits are the same.  The step is
+// memory bound; 8-byte accesses halve its load and store instructions (4096^2
+// TRT step with moments 222.5 -> 219.7 us, 6.4 TB/s).
+template <bool TRT, typename I>
+__global__ void __launch_bounds__(BX) fused2_k(float *__restrict__ fo, const float *__restrict__ fi,
+                                                float *__restrict__ rho, float *__restrict__ ux,
+                                                float *__restrict__ uy, const uint8_t *__restrict__ solid,
+                                                int Nx, int Ny, unsigned magic, float s1, float s2) {
+    int i, j;
+    if (!node_ij(Nx / 2, Ny, magic, i, j)) return;
+    i *= 2;
+    const I P = (I)Nx * (I)Ny, c = (I)i + (I)Nx * (I)j;
+    Lanes2 p[9];
+    pull_bb_pair<I>(fi, Nx, Ny, P, c, i, j, p);
+    const uchar2 sd = solid ? *reinterpret_cast<const uchar2 *>(solid + c) : make_uchar2(0, 0);
+    float2 m[3];
+    const auto node = [&](float *v, bool is_solid, float &r, float &a, float &b) {
+        if (is_solid) {
+            swap_pairs(v);
+            r = 1.0f; a = 0.0f; b = 0.0f;
+        } else if (TRT) {
+            trt_node(v, s1, s2, r, a, b);
+        } else {
+            bgk(v, s1, r, a, b);
+        }
+    };
+    float x[9], y[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) { x[q] = p[q].v.x; y[q] = p[q].v.y; }
+    node(x, sd.x, m[0].x, m[1].x, m[2].x);
+    node(y, sd.y, m[0].y, m[1].y, m[2].y);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) *reinterpret_cast<float2 *>(fo + c + q * P) = make_float2(x[q], y[q]);
+    *reinterpret_cast<float2 *>(rho + c) = m[0];
+    *reinterpret_cast<float2 *>(ux + c) = m[1];
+    *reinterpret_cast<float2 *>(uy + c) = m[2];
+}
+
+// natconv_k in FP32 for even Nx and 8-byte aligned arrays: two adjacent nodes
+// per thread as two lanes (Lanes2), each evaluating natconv_k's expression
+// tree with packed round-to-nearest adds and multiplies, to within the few
+// ulp that Lanes2 states.  natconv_k is bound by its instructions (about 350
+// separate adds and multiplies per node, both lattices of a 512^2 grid in L2);
+// the packed form issues half of them (512^2: 9.0 -> 7.5 us per step of a
+// captured loop).
+template <bool VT, typename I>
+__global__ void __launch_bounds__(BX) natconv2_k(float *__restrict__ fo, const float *__restrict__ fi,
+                                                  float *__restrict__ go, const float *__restrict__ gi,
+                                                  float *__restrict__ Temp, int Nx, int Ny, float w_f,
+                                                  float w_T, float beta_g, float T_ref, float T_hot,
+                                                  float T_cold, float nu_ref, float T0_visc,
+                                                  float a_visc, unsigned magic) {
+    int i, j;
+    if (!node_ij(Nx / 2, Ny, magic, i, j)) return;
+    i *= 2;
+    const I P = (I)Nx * (I)Ny, c = (I)i + (I)Nx * (I)j;
+    const auto sp = [](float x) { return Lanes2::of(make_float2(x, x)); };
+    Lanes2 fp[9], gp[9];
+    pull_bb_pair<I>(fi, Nx, Ny, P, c, i, j, fp);
+    pull_bb_pair<I>(gi, Nx, Ny, P, c, i, j, gp);
+    const float h1 = 2.0f * (float)(1.0 / 9.0), h5 = 2.0f * (float)(1.0 / 36.0);
+    if (i == 0) {
+        gp[1].v.x = -gp[1].v.x + h1 * T_hot;
+        gp[5].v.x = -gp[5].v.x + h5 * T_hot;
+        gp[8].v.x = -gp[8].v.x + h5 * T_hot;
+    }
+    if (i + 1 == Nx - 1) {
+        gp[3].v.y = -gp[3].v.y + h1 * T_cold;
+        gp[6].v.y = -gp[6].v.y + h5 * T_cold;
+        gp[7].v.y = -gp[7].v.y + h5 * T_cold;
+    }
+    const Lanes2 Tl = gp[0] + gp[1] + gp[2] + gp[3] + gp[4] + gp[5] + gp[6] + gp[7] + gp[8];
+    *reinterpret_cast<float2 *>(Temp + c) = Tl.v;
+    const Lanes2 fy = sp(beta_g) * (Tl - sp(T_ref));
+    const Lanes2 rho = fp[0] + fp[1] + fp[2] + fp[3] + fp[4] + fp[5] + fp[6] + fp[7] + fp[8];
+    const Lanes2 inv = Lanes2(1.0) / rho;
+    const Lanes2 ux = (fp[1] - fp[3] + fp[5] - fp[6] - fp[7] + fp[8]) * inv;
+    const Lanes2 uy = ((fp[2] - fp[4] + fp[5] + fp[6] - fp[7] - fp[8]) + fy / Lanes2(2.0)) * inv;
+    collide_thermal(gp, ux, uy, sp(w_T));
+#pragma unroll
+    for (int q = 0; q < 9; ++q) *reinterpret_cast<float2 *>(go + c + q * P) = gp[q].v;
+    Lanes2 w = sp(w_f);
+    if (VT) {
+        const auto rate = [&](float T) {
+            const float nul = nu_ref * kb_exp(a_visc * (T - T0_visc));
+            return 1.0f / (3.0f * nul + 0.5f);
+        };
+        w.v = make_float2(rate(Tl.v.x), rate(Tl.v.y));
+    }
+    collide_guo(fp, rho, ux, uy, Lanes2(0.0), fy, w);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) *reinterpret_cast<float2 *>(fo + c + q * P) = fp[q].v;
+}
+
 // compute_temperature_2d!: src/kernels/thermal_2d.jl:113-138
 template <typename T>
 __global__ void __launch_bounds__(BX) temperature_k(T *__restrict__ Temp, const T *__restrict__ gg,
@@ -1160,6 +1287,55 @@ void launch_forced_2d(T *f, const T *Temp, const uint8_t *solid, const T *Fxf, c
         guo_k<T, true><<<nodes_grid(Nx, Ny), BX, 0, s>>>(f, solid, Fxf, Fyf, g, omega, T(0), T(0));
 }
 
+// Fused BGK / TRT step: FP32 on even Nx with 8-byte aligned arrays (the solid
+// mask 2-byte) takes two nodes per thread, everything else one.
+template <bool TRT, typename T>
+void launch_fused(T *fo, const T *fi, T *rho, T *ux, T *uy, const uint8_t *solid, int Nx, int Ny, T s1,
+                  T s2, cudaStream_t s) {
+    if constexpr (sizeof(T) == 4) {
+        const auto al = [](const void *q, uintptr_t n) { return ((uintptr_t)q & (n - 1)) == 0; };
+        if (Nx % 2 == 0 && al(fo, 8) && al(fi, 8) && al(rho, 8) && al(ux, 8) && al(uy, 8) && al(solid, 2)) {
+            const unsigned magic = kb::node_magic(Nx / 2, Ny);
+            const dim3 grid = nodes_grid(Nx / 2, Ny);
+            if (10.0 * (double)Nx * (double)Ny < 2147483647.0)
+                fused2_k<TRT, int><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, solid, Nx, Ny, magic, s1, s2);
+            else
+                fused2_k<TRT, long long><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, solid, Nx, Ny, magic, s1, s2);
+            return;
+        }
+    }
+    if constexpr (TRT)
+        fused_trt_k<T><<<nodes_grid(Nx, Ny), BX, 0, s>>>(fo, fi, rho, ux, uy, solid, grid2<T>(Nx, Ny), s1, s2);
+    else
+        fused_bgk_k<T><<<nodes_grid(Nx, Ny), BX, 0, s>>>(fo, fi, rho, ux, uy, solid, grid2<T>(Nx, Ny), s1);
+}
+
+// Fused natural convection: FP32 on even Nx with 8-byte aligned arrays takes
+// two nodes per thread (natconv2_k), everything else one.
+template <typename T, bool VT>
+void launch_natconv(T *fo, const T *fi, T *go, const T *gi, T *Temp, int Nx, int Ny, T w_f, T w_T,
+                    T beta_g, T T_ref, T T_hot, T T_cold, T nu_ref, T T0_visc, T a_visc,
+                    cudaStream_t s) {
+    const Grid2<T> g = grid2<T>(Nx, Ny);
+    if constexpr (sizeof(T) == 4) {
+        const auto al = [](const void *q) { return ((uintptr_t)q & 7) == 0; };
+        if (Nx % 2 == 0 && al(fo) && al(fi) && al(go) && al(gi) && al(Temp)) {
+            const unsigned magic = kb::node_magic(Nx / 2, Ny);
+            const dim3 grid = nodes_grid(Nx / 2, Ny);
+            if (10.0 * (double)g.plane < 2147483647.0)
+                natconv2_k<VT, int><<<grid, BX, 0, s>>>(fo, fi, go, gi, Temp, Nx, Ny, w_f, w_T, beta_g,
+                                                        T_ref, T_hot, T_cold, nu_ref, T0_visc, a_visc, magic);
+            else
+                natconv2_k<VT, long long><<<grid, BX, 0, s>>>(fo, fi, go, gi, Temp, Nx, Ny, w_f, w_T,
+                                                              beta_g, T_ref, T_hot, T_cold, nu_ref,
+                                                              T0_visc, a_visc, magic);
+            return;
+        }
+    }
+    natconv_k<T, VT><<<nodes_grid(Nx, Ny), BX, 0, s>>>(fo, fi, go, gi, Temp, g, w_f, w_T, beta_g, T_ref,
+                                                       T_hot, T_cold, nu_ref, T0_visc, a_visc);
+}
+
 int check_dims(const char *what, int Nx, int Ny) {
     if (Nx < 1 || Ny < 1 || Ny > 65535)
         return kb::set_error(KB_ERR_ARG, "%s: bad grid %d x %d (need Nx >= 1, 1 <= Ny <= 65535)",
@@ -1305,9 +1481,8 @@ int kb_fused_bgk_step(void *f_out, const void *f_in, void *rho, void *ux, void *
     KB_REQUIRE(f_out != f_in, "kb_fused_bgk_step: f_out and f_in must differ");
     if (int e = check_dims("kb_fused_bgk_step", Nx, Ny)) return e;
     KB_DISPATCH_PLAIN("kb_fused_bgk_step", dtype,
-        (fused_bgk_k<T><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
-            (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
-            (T)omega)));
+        (launch_fused<false, T>((T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, Nx, Ny,
+                                (T)omega, T(0), kb::as_stream(stream))));
 }
 
 int kb_trt_rates(double nu, double Lambda, double *s_plus, double *s_minus) {
@@ -1329,9 +1504,8 @@ int kb_fused_trt_step(void *f_out, const void *f_in, void *rho, void *ux, void *
     double sp, sm;
     if (int e = kb_trt_rates(nu, Lambda, &sp, &sm)) return e;
     KB_DISPATCH_PLAIN("kb_fused_trt_step", dtype,
-        (fused_trt_k<T><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
-            (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
-            (T)sp, (T)sm)));
+        (launch_fused<true, T>((T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, Nx, Ny,
+                               (T)sp, (T)sm, kb::as_stream(stream))));
 }
 
 int kb_fused_trt_libb_step(void *f_out, const void *f_in, void *rho, void *ux, void *uy,
@@ -1507,10 +1681,9 @@ int kb_fused_natconv_step(void *f_out, const void *f_in, void *g_out, const void
                                           Ny, omega_f, omega_T, beta_g, T_ref_buoy, T_hot, T_cold,
                                           0.0, 0.0, 0.0, kb::as_stream(stream));
     KB_DISPATCH_PLAIN("kb_fused_natconv_step", dtype,
-        (natconv_k<T, false><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
-            (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, (T *)Temp, grid2<T>(Nx, Ny),
-            (T)omega_f, (T)omega_T, (T)beta_g, (T)T_ref_buoy, (T)T_hot, (T)T_cold, T(0), T(0),
-            T(0))));
+        (launch_natconv<T, false>((T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, (T *)Temp, Nx,
+                                  Ny, (T)omega_f, (T)omega_T, (T)beta_g, (T)T_ref_buoy, (T)T_hot,
+                                  (T)T_cold, T(0), T(0), T(0), kb::as_stream(stream))));
 }
 
 int kb_fused_natconv_vt_step(void *f_out, const void *f_in, void *g_out, const void *g_in,
@@ -1525,10 +1698,9 @@ int kb_fused_natconv_vt_step(void *f_out, const void *f_in, void *g_out, const v
                                           Ny, 0.0, omega_T, beta_g, T_ref_buoy, T_hot, T_cold,
                                           nu_ref, T0_visc, alpha_visc, kb::as_stream(stream));
     KB_DISPATCH_PLAIN("kb_fused_natconv_vt_step", dtype,
-        (natconv_k<T, true><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
-            (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, (T *)Temp, grid2<T>(Nx, Ny),
-            T(0), (T)omega_T, (T)beta_g, (T)T_ref_buoy, (T)T_hot, (T)T_cold, (T)nu_ref,
-            (T)T0_visc, (T)alpha_visc)));
+        (launch_natconv<T, true>((T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, (T *)Temp, Nx,
+                                 Ny, T(0), (T)omega_T, (T)beta_g, (T)T_ref_buoy, (T)T_hot, (T)T_cold,
+                                 (T)nu_ref, (T)T0_visc, (T)alpha_visc, kb::as_stream(stream))));
 }
 
 int kb_compute_temperature_2d(void *Temp, const void *g, int Nx, int Ny, int dtype, void *stream) {

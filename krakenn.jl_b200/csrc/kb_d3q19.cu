@@ -146,6 +146,26 @@ __global__ void __launch_bounds__(BX) macroscopic_forced_k(T *__restrict__ rho, 
     uz[c] = ((p[5] - p[6] + p[11] + p[12] - p[13] - p[14] + p[15] + p[16] - p[17] - p[18]) + fz / T(2)) * inv;
 }
 
+// TRT update of one fluid node in place (CollideTRTDirect_3D), with its moments.
+template <typename T>
+__device__ __forceinline__ void trt_node(T *p, T sp, T sm, T &r, T &ux, T &uy, T &uz) {
+    T feq[19];
+    moments(p, r, ux, uy, uz);
+    const T usq = ux * ux + uy * uy + uz * uz;
+    feq_all(r, ux, uy, uz, usq, feq);
+    const T a = (sp + sm) * T(0.5), b = (sp - sm) * T(0.5);
+    const int pa[9] = {1, 3, 5, 7, 8, 11, 12, 15, 16};
+    const int pb[9] = {2, 4, 6, 10, 9, 14, 13, 18, 17};
+    p[0] = p[0] - sp * (p[0] - feq[0]);
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+        const int x = pa[m], y = pb[m];
+        const T fx = p[x], fy = p[y];
+        p[x] = fx - a * (fx - feq[x]) - b * (fy - feq[y]);
+        p[y] = fy - a * (fy - feq[y]) - b * (fx - feq[x]);
+    }
+}
+
 // Fused TRT step with the reference arithmetic (PullHalfwayBB_3D +
 // SolidInert_3D + Moments_3D + CollideTRTDirect_3D + WriteMoments_3D,
 // src/kernels/dsl/bricks_3d.jl:64-230, 476-483).  I: element-offset type.
@@ -288,6 +308,82 @@ __global__ void __launch_bounds__(BX) fused_trt_links_k(T *__restrict__ fo, cons
     } else {
         trt_links_node<T, I>(fo, fi, rho, ux, uy, uz, L, g, sp, sm, c, i, j, k, cl);
     }
+}
+
+// FP32 with even Nx and 8-byte aligned arrays: two adjacent nodes per thread,
+// each with the one-node kernel's scalar arithmetic, so the bits are the same.
+// CLS = false is fused_trt_k (cls: the solid mask or null), CLS = true is
+// fused_trt_links_k<SKIP_CUT> (cls: the table's class bytes; class 2 nodes are
+// left to fused_trt_cut_k).  Memory bound: the 8-byte accesses halve the
+// stores and take a third off the loads (192^3 cut-link step 197.5 -> 188.5
+// us, 5.7 TB/s).
+template <bool CLS, typename I>
+__global__ void __launch_bounds__(BX) fused_trt2_k(float *__restrict__ fo, const float *__restrict__ fi,
+                                                    float *__restrict__ rho, float *__restrict__ ux,
+                                                    float *__restrict__ uy, float *__restrict__ uz,
+                                                    const uint8_t *__restrict__ cls, Grid3 g,
+                                                    unsigned magic, float sp, float sm) {
+    int i, j;
+    const int k = blockIdx.z;
+    if (!node_ij(g.Nx / 2, g.Ny, magic, i, j)) return;
+    i *= 2;
+    const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
+    const I P = (I)g.plane;
+    float x[19], y[19];
+    pull19_pair<I>(fi + c, P, g, i, j, k, x, y);
+    const uchar2 cl = cls ? *reinterpret_cast<const uchar2 *>(cls + c) : make_uchar2(0, 0);
+    float2 m[4];
+    const auto node = [&](float *v, bool is_solid, float &r, float &a, float &b, float &d) {
+        if (is_solid) {
+            feq_all(1.0f, 0.0f, 0.0f, 0.0f, 0.0f, v);
+            r = 1.0f; a = 0.0f; b = 0.0f; d = 0.0f;
+        } else {
+            trt_node(v, sp, sm, r, a, b, d);
+        }
+    };
+    node(x, CLS ? cl.x == 1 : cl.x != 0, m[0].x, m[1].x, m[2].x, m[3].x);
+    node(y, CLS ? cl.y == 1 : cl.y != 0, m[0].y, m[1].y, m[2].y, m[3].y);
+    float *__restrict__ o0 = fo + c;
+    if (CLS && (cl.x == 2 || cl.y == 2)) {
+        // one or both nodes belong to the cut-node kernel
+        if (cl.x != 2) {
+#pragma unroll
+            for (int q = 0; q < 19; ++q) o0[q * P] = x[q];
+            if (rho) { rho[c] = m[0].x; ux[c] = m[1].x; uy[c] = m[2].x; uz[c] = m[3].x; }
+        }
+        if (cl.y != 2) {
+#pragma unroll
+            for (int q = 0; q < 19; ++q) o0[q * P + 1] = y[q];
+            if (rho) { rho[c + 1] = m[0].y; ux[c + 1] = m[1].y; uy[c + 1] = m[2].y; uz[c + 1] = m[3].y; }
+        }
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < 19; ++q) *reinterpret_cast<float2 *>(o0 + q * P) = make_float2(x[q], y[q]);
+    if (rho) {
+        *reinterpret_cast<float2 *>(rho + c) = m[0];
+        *reinterpret_cast<float2 *>(ux + c) = m[1];
+        *reinterpret_cast<float2 *>(uy + c) = m[2];
+        *reinterpret_cast<float2 *>(uz + c) = m[3];
+    }
+}
+
+// Whether fused_trt2_k takes these arrays.
+inline bool pairs_fit(const Grid3 &g, const void *fo, const void *fi, const void *rho, const void *ux,
+                      const void *uy, const void *uz, const void *cls) {
+    const auto al = [](const void *q, uintptr_t n) { return ((uintptr_t)q & (n - 1)) == 0; };
+    return g.Nx % 2 == 0 && al(fo, 8) && al(fi, 8) && al(rho, 8) && al(ux, 8) && al(uy, 8) && al(uz, 8) &&
+           al(cls, 2);
+}
+
+template <bool CLS>
+void launch_trt2(float *fo, const float *fi, float *rho, float *ux, float *uy, float *uz,
+                 const uint8_t *cls, const Grid3 &g, float sp, float sm, cudaStream_t s) {
+    if (offsets_fit_int(g, 19))
+        fused_trt2_k<CLS, int><<<pair_grid(g), BX, 0, s>>>(fo, fi, rho, ux, uy, uz, cls, g, pair_magic(g), sp, sm);
+    else
+        fused_trt2_k<CLS, long long><<<pair_grid(g), BX, 0, s>>>(fo, fi, rho, ux, uy, uz, cls, g,
+                                                                 pair_magic(g), sp, sm);
 }
 
 // The cut nodes (class 2) of a compact table, one thread per record.
@@ -763,6 +859,52 @@ __global__ void __launch_bounds__(BX) cavity_step_k(T *__restrict__ fo, const T 
     }
 }
 
+// cavity_step_k in FP32 for even Nx and 8-byte aligned arrays: two adjacent
+// nodes per thread with its scalar arithmetic (same bits), 8-byte accesses.
+template <typename I>
+__global__ void __launch_bounds__(BX) cavity_step2_k(float *__restrict__ fo, const float *__restrict__ fi,
+                                                      float *__restrict__ rho, float *__restrict__ ux,
+                                                      float *__restrict__ uy, float *__restrict__ uz,
+                                                      const uint8_t *__restrict__ solid, Grid3 g,
+                                                      unsigned magic, float omega, float u_lid) {
+    int i, j;
+    const int k = blockIdx.z;
+    if (!node_ij(g.Nx / 2, g.Ny, magic, i, j)) return;
+    i *= 2;
+    const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
+    const I P = (I)g.plane;
+    float x[19], y[19];
+    pull19_pair<I>(fi + c, P, g, i, j, k, x, y);
+    const uchar2 sd = solid ? *reinterpret_cast<const uchar2 *>(solid + c) : make_uchar2(0, 0);
+    const auto node = [&](float *v, bool is_solid) {
+        if (k == g.Nz - 1) zou_he_top_node(v, u_lid);
+        if (is_solid) {
+            swap_pairs(v);
+            return;
+        }
+        float r, a, b, d, feq[19];
+        moments(v, r, a, b, d);
+        const float usq = a * a + b * b + d * d;
+        feq_all(r, a, b, d, usq, feq);
+#pragma unroll
+        for (int q = 0; q < 19; ++q) v[q] = v[q] - omega * (v[q] - feq[q]);
+    };
+    node(x, sd.x);
+    node(y, sd.y);
+    float *__restrict__ o0 = fo + c;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) *reinterpret_cast<float2 *>(o0 + q * P) = make_float2(x[q], y[q]);
+    if (rho) {
+        float2 r, a, b, d;
+        moments(x, r.x, a.x, b.x, d.x);
+        moments(y, r.y, a.y, b.y, d.y);
+        *reinterpret_cast<float2 *>(rho + c) = r;
+        *reinterpret_cast<float2 *>(ux + c) = a;
+        *reinterpret_cast<float2 *>(uy + c) = b;
+        *reinterpret_cast<float2 *>(uz + c) = d;
+    }
+}
+
 // One step of run_natural_convection_3d (src/drivers/thermal.jl:455-537) in
 // one launch: stream f and g, hot west / cold east anti-bounce-back faces,
 // temperature, moments (without the half force), thermal BGK, Boussinesq BGK
@@ -970,6 +1112,13 @@ int kb_cavity_step_3d(void *f_out, const void *f_in, void *rho, void *ux, void *
     if (int e = check_dims(what, Nx, Ny, Nz)) return e;
     const Grid3 g = grid3(Nx, Ny, Nz);
     cudaStream_t s = kb::as_stream(stream);
+    if (dtype == KB_F32 && pairs_fit(g, f_out, f_in, rho, ux, uy, uz, is_solid)) {
+        const auto k2 = offsets_fit_int(g, 19) ? cavity_step2_k<int> : cavity_step2_k<long long>;
+        k2<<<pair_grid(g), BX, 0, s>>>((float *)f_out, (const float *)f_in, (float *)rho, (float *)ux,
+                                       (float *)uy, (float *)uz, is_solid, g, pair_magic(g), (float)omega,
+                                       (float)u_lid);
+        return kb::check_launch(what);
+    }
     KB3_DISPATCH_PLAIN(what, dtype,
         if (offsets_fit_int(g, 19))
             (cavity_step_k<T, int><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
@@ -1038,7 +1187,10 @@ int trt3d_step(const char *what, void *f_out, const void *f_in, void *rho, void 
                 (double *)f_out, (const double *)f_in, (double *)rho, (double *)ux, (double *)uy,
                 (double *)uz, is_solid, g, sp, sm);
     } else if (dtype == KB_F32) {
-        if (i32)
+        if (pairs_fit(g, f_out, f_in, rho, ux, uy, uz, is_solid))
+            launch_trt2<false>((float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
+                               (float *)uz, is_solid, g, (float)sp, (float)sm, s);
+        else if (i32)
             fused_trt_k<float, int><<<grid, BX, 0, s>>>(
                 (float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
                 (float *)uz, is_solid, g, (float)sp, (float)sm);
@@ -1413,7 +1565,12 @@ int launch_links_3d_i(T *fo, const T *fi, T *rho, T *ux, T *uy, T *uz,
         cudaGetLastError();
     const unsigned nb = (unsigned)((L.n_rec + BX - 1) / BX);
     fused_trt_cut_k<T, I><<<nb, BX, 0, cs>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
-    fused_trt_links_k<T, I, true><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
+    bool pairs = false;
+    if constexpr (sizeof(T) == 4) {
+        pairs = pairs_fit(g, fo, fi, rho, ux, uy, uz, L.cls);
+        if (pairs) launch_trt2<true>(fo, fi, rho, ux, uy, uz, L.cls, g, sp, sm, s);
+    }
+    if (!pairs) fused_trt_links_k<T, I, true><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
     if (cs != s && (cudaEventRecord(ss->join, cs) != cudaSuccess || cudaStreamWaitEvent(s, ss->join, 0) != cudaSuccess))
         return kb::set_error(KB_ERR_CUDA, "kb_fused_trt_libb_links_step_3d: joining the cut-node stream failed");
     return KB_OK;

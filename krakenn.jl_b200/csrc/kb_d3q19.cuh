@@ -87,6 +87,37 @@ __device__ __forceinline__ void pull19_at(const R *__restrict__ f0, I P, const P
     p[18] = ld(f0[(s.yp && s.zp) ? s.dyp + s.dzp + 18 * P : 15 * P]);
 }
 
+// Pull of the adjacent nodes (i, j, k) and (i + 1, j, k), i even, even Nx,
+// 8-byte aligned planes: the values pull19_at gives for each.  A population
+// without an x component is one 8-byte load.
+template <typename I>
+__device__ __forceinline__ void pull19_pair(const float *__restrict__ f0, I P, const Grid3 &g, int i, int j,
+                                            int k, float *a, float *b) {
+    const Pull3<I> s = pull_geometry<I>(g, i, j, k);
+    const bool px = g.per & 1;
+    const bool xp = px || i + 1 < g.Nx - 1;                          // of node i + 1
+    const I dxp = i + 1 < g.Nx - 1 ? (I)1 : -(I)(g.Nx - 1);
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        const int cx = cx19(q), cy = cy19(q), cz = cz19(q);
+        const bool ok = (cy == 0 || (cy > 0 ? s.ym : s.yp)) && (cz == 0 || (cz > 0 ? s.zm : s.zp));
+        const I d = (cy == 0 ? (I)0 : (cy > 0 ? s.dym : s.dyp)) + (cz == 0 ? (I)0 : (cz > 0 ? s.dzm : s.dzp)) +
+                    (I)q * P;
+        const I o = (I)opp19(q) * P;
+        if (cx == 0) {
+            const float2 v = *reinterpret_cast<const float2 *>(f0 + (ok ? d : o));
+            a[q] = v.x;
+            b[q] = v.y;
+        } else if (cx > 0) {
+            a[q] = f0[(ok && s.xm) ? d + s.dxm : o];
+            b[q] = f0[ok ? d : o + 1];
+        } else {
+            a[q] = f0[ok ? d + 1 : o];
+            b[q] = f0[(ok && xp) ? d + 1 + dxp : o + 1];
+        }
+    }
+}
+
 // Pull with 64-bit offsets from the buffer base f and node index c.
 template <typename R, typename V, typename Load>
 __device__ __forceinline__ void pull19(const R *__restrict__ f, size_t P, size_t c,
@@ -103,6 +134,12 @@ inline bool offsets_fit_int(const Grid3 &g, int Q) {
 // Launch grid of the one-node kernels on grid g (NODE3), BX threads a block.
 inline dim3 node_grid(const Grid3 &g) {
     return dim3(node_blocks(g.Nx, g.Ny, g.magic), g.magic ? 1 : g.Ny, g.Nz);
+}
+// ... and of the kernels with two adjacent nodes per thread (even Nx).
+inline unsigned pair_magic(const Grid3 &g) { return node_magic(g.Nx / 2, g.Ny); }
+inline dim3 pair_grid(const Grid3 &g) {
+    const unsigned m = pair_magic(g);
+    return dim3(node_blocks(g.Nx / 2, g.Ny, m), m ? 1 : g.Ny, g.Nz);
 }
 static_assert(BX == NODE_BX, "one-node kernels number nodes in blocks of NODE_BX");
 
