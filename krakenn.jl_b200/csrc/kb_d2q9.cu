@@ -306,6 +306,9 @@ __global__ void __launch_bounds__(BX) fused_bgk_k(T *__restrict__ fo, const T *_
                                                    const uint8_t *__restrict__ solid, Grid2<T> g,
                                                    T omega) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     T p[9];
     pull_bb(fi, g, i, j, p);
     T r, a, b;
@@ -348,6 +351,9 @@ __global__ void __launch_bounds__(BX) fused_trt_k(T *__restrict__ fo, const T *_
                                                    const uint8_t *__restrict__ solid, Grid2<T> g,
                                                    T sp, T sm) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     T p[9];
     pull_bb(fi, g, i, j, p);
     T r, a_, b_;
@@ -594,6 +600,9 @@ __global__ void __launch_bounds__(BX) cavity_mrt_step_k(T *__restrict__ fo, cons
                                                          Grid2<T> g, T s_e, T s_eps, T s_q,
                                                          T s_nu, T u_lid) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     T p[9];
     pull_bb(fi, g, i, j, p);
     if (j == g.Ny - 1) zou_he_north_node(p, u_lid);
@@ -685,6 +694,9 @@ __global__ void __launch_bounds__(BX) cavity_step_k(T *__restrict__ fo, const T 
                                                      const uint8_t *__restrict__ solid, Grid2<T> g,
                                                      T omega, T u_lid) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     T p[9];
     pull_bb(fi, g, i, j, p);
     if (j == g.Ny - 1) zou_he_north_node(p, u_lid);
@@ -714,6 +726,9 @@ __global__ void __launch_bounds__(BX) cavity_movingwall_k(T *__restrict__ fo, co
                                                            const uint8_t *__restrict__ solid,
                                                            Grid2<T> g, T omega, T u_lid) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     T p[9];
     pull_bb(fi, g, i, j, p);
     T r, a, b;
@@ -802,6 +817,9 @@ __global__ void __launch_bounds__(BX) natconv_k(T *__restrict__ fo, const T *__r
                                                  T beta_g, T T_ref, T T_hot, T T_cold, T nu_ref,
                                                  T T0_visc, T a_visc) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    gi = pdl_fresh(gi);
     T fp[9], gp[9];
     pull_bb(fi, g, i, j, fp);
     pull_bb(gi, g, i, j, gp);
@@ -863,6 +881,9 @@ __global__ void __launch_bounds__(BX) fused2_k(float *__restrict__ fo, const flo
     int i, j;
     if (!node_ij(Nx / 2, Ny, magic, i, j)) return;
     i *= 2;
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     const I P = (I)Nx * (I)Ny, c = (I)i + (I)Nx * (I)j;
     Lanes2 p[9];
     pull_bb_pair<I>(fi, Nx, Ny, P, c, i, j, p);
@@ -907,6 +928,9 @@ __global__ void __launch_bounds__(BX) natconv2_k(float *__restrict__ fo, const f
     int i, j;
     if (!node_ij(Nx / 2, Ny, magic, i, j)) return;
     i *= 2;
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    gi = pdl_fresh(gi);
     const I P = (I)Nx * (I)Ny, c = (I)i + (I)Nx * (I)j;
     const auto sp = [](float x) { return Lanes2::of(make_float2(x, x)); };
     Lanes2 fp[9], gp[9];
@@ -1097,6 +1121,9 @@ __global__ void __launch_bounds__(BX) rayleigh_step_k(T *__restrict__ fo, const 
                                                        Grid2<T> g, T w_f, T w_T, T beta_g, T T_ref,
                                                        T T_lo, T T_hi) {
     NODE2
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    gi = pdl_fresh(gi);
     T p[9], h[9];
     if (XPER) {
         pull_px_wy(gi, g, i, j, h);
@@ -1298,16 +1325,16 @@ void launch_fused(T *fo, const T *fi, T *rho, T *ux, T *uy, const uint8_t *solid
             const unsigned magic = kb::node_magic(Nx / 2, Ny);
             const dim3 grid = nodes_grid(Nx / 2, Ny);
             if (10.0 * (double)Nx * (double)Ny < 2147483647.0)
-                fused2_k<TRT, int><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, solid, Nx, Ny, magic, s1, s2);
+                kb::launch_pdl(fused2_k<TRT, int>, grid, dim3(BX), s, fo, fi, rho, ux, uy, solid, Nx, Ny, magic, s1, s2);
             else
-                fused2_k<TRT, long long><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, solid, Nx, Ny, magic, s1, s2);
+                kb::launch_pdl(fused2_k<TRT, long long>, grid, dim3(BX), s, fo, fi, rho, ux, uy, solid, Nx, Ny, magic, s1, s2);
             return;
         }
     }
     if constexpr (TRT)
-        fused_trt_k<T><<<nodes_grid(Nx, Ny), BX, 0, s>>>(fo, fi, rho, ux, uy, solid, grid2<T>(Nx, Ny), s1, s2);
+        kb::launch_pdl(fused_trt_k<T>, nodes_grid(Nx, Ny), dim3(BX), s, fo, fi, rho, ux, uy, solid, grid2<T>(Nx, Ny), s1, s2);
     else
-        fused_bgk_k<T><<<nodes_grid(Nx, Ny), BX, 0, s>>>(fo, fi, rho, ux, uy, solid, grid2<T>(Nx, Ny), s1);
+        kb::launch_pdl(fused_bgk_k<T>, nodes_grid(Nx, Ny), dim3(BX), s, fo, fi, rho, ux, uy, solid, grid2<T>(Nx, Ny), s1);
 }
 
 // Fused natural convection: FP32 on even Nx with 8-byte aligned arrays takes
@@ -1323,16 +1350,16 @@ void launch_natconv(T *fo, const T *fi, T *go, const T *gi, T *Temp, int Nx, int
             const unsigned magic = kb::node_magic(Nx / 2, Ny);
             const dim3 grid = nodes_grid(Nx / 2, Ny);
             if (10.0 * (double)g.plane < 2147483647.0)
-                natconv2_k<VT, int><<<grid, BX, 0, s>>>(fo, fi, go, gi, Temp, Nx, Ny, w_f, w_T, beta_g,
+                kb::launch_pdl(natconv2_k<VT, int>, grid, dim3(BX), s, fo, fi, go, gi, Temp, Nx, Ny, w_f, w_T, beta_g,
                                                         T_ref, T_hot, T_cold, nu_ref, T0_visc, a_visc, magic);
             else
-                natconv2_k<VT, long long><<<grid, BX, 0, s>>>(fo, fi, go, gi, Temp, Nx, Ny, w_f, w_T,
+                kb::launch_pdl(natconv2_k<VT, long long>, grid, dim3(BX), s, fo, fi, go, gi, Temp, Nx, Ny, w_f, w_T,
                                                               beta_g, T_ref, T_hot, T_cold, nu_ref,
                                                               T0_visc, a_visc, magic);
             return;
         }
     }
-    natconv_k<T, VT><<<nodes_grid(Nx, Ny), BX, 0, s>>>(fo, fi, go, gi, Temp, g, w_f, w_T, beta_g, T_ref,
+    kb::launch_pdl(natconv_k<T, VT>, nodes_grid(Nx, Ny), dim3(BX), s, fo, fi, go, gi, Temp, g, w_f, w_T, beta_g, T_ref,
                                                        T_hot, T_cold, nu_ref, T0_visc, a_visc);
 }
 
@@ -1593,7 +1620,7 @@ int kb_cavity_step_2d(void *f_out, const void *f_in, void *rho, void *ux, void *
     KB_REQUIRE(f_out != f_in, "kb_cavity_step_2d: f_out and f_in must differ");
     if (int e = check_dims("kb_cavity_step_2d", Nx, Ny)) return e;
     KB_DISPATCH_PLAIN("kb_cavity_step_2d", dtype,
-        (cavity_step_k<T><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
+        (kb::launch_pdl(cavity_step_k<T>, nodes_grid(Nx, Ny), dim3(BX), kb::as_stream(stream),
             (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
             (T)omega, (T)u_lid)));
 }
@@ -1609,7 +1636,7 @@ int kb_cavity_mrt_step_2d(void *f_out, const void *f_in, void *rho, void *ux, vo
     if (int e = check_dims("kb_cavity_mrt_step_2d", Nx, Ny)) return e;
     const double s_nu = 1.0 / (3.0 * nu + 0.5);
     KB_DISPATCH_PLAIN("kb_cavity_mrt_step_2d", dtype,
-        (cavity_mrt_step_k<T><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
+        (kb::launch_pdl(cavity_mrt_step_k<T>, nodes_grid(Nx, Ny), dim3(BX), kb::as_stream(stream),
             (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
             (T)s_e, (T)s_eps, (T)s_q, (T)s_nu, (T)u_lid)));
 }
@@ -1644,7 +1671,7 @@ int kb_cavity_movingwall_step_2d(void *f_out, const void *f_in, void *rho, void 
     KB_REQUIRE(nm == 0 || nm == 3, "kb_cavity_movingwall_step_2d: pass all three moment arrays or none");
     if (int e = check_dims("kb_cavity_movingwall_step_2d", Nx, Ny)) return e;
     KB_DISPATCH_PLAIN("kb_cavity_movingwall_step_2d", dtype,
-        (cavity_movingwall_k<T><<<nodes_grid(Nx, Ny), BX, 0, kb::as_stream(stream)>>>(
+        (kb::launch_pdl(cavity_movingwall_k<T>, nodes_grid(Nx, Ny), dim3(BX), kb::as_stream(stream),
             (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
             (T)omega, (T)u_lid)));
 }
@@ -1660,12 +1687,12 @@ int kb_rayleigh_step_2d(void *f_out, const void *f_in, void *g_out, const void *
     cudaStream_t s = kb::as_stream(stream);
     KB_DISPATCH_PLAIN(what, dtype,
         if (vertical)
-            (rayleigh_step_k<T, true><<<nodes_grid(Nx, Ny), BX, 0, s>>>(
-                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, grid2<T>(Nx, Ny), (T)omega_f,
+            (kb::launch_pdl(rayleigh_step_k<T, true>, nodes_grid(Nx, Ny), dim3(BX), s,
+            (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, grid2<T>(Nx, Ny), (T)omega_f,
                 (T)omega_T, (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold));
         else
-            (rayleigh_step_k<T, false><<<nodes_grid(Nx, Ny), BX, 0, s>>>(
-                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, grid2<T>(Nx, Ny), (T)omega_f,
+            (kb::launch_pdl(rayleigh_step_k<T, false>, nodes_grid(Nx, Ny), dim3(BX), s,
+            (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, grid2<T>(Nx, Ny), (T)omega_f,
                 (T)omega_T, (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold)));
 }
 

@@ -176,6 +176,9 @@ __global__ void __launch_bounds__(BX) fused_trt_k(T *__restrict__ fo, const T *_
                                                    const uint8_t *__restrict__ solid, Grid3 g, T sp,
                                                    T sm) {
     NODE3_IJK
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     T *__restrict__ o0 = fo + c;
@@ -327,6 +330,9 @@ __global__ void __launch_bounds__(BX) fused_trt2_k(float *__restrict__ fo, const
     const int k = blockIdx.z;
     if (!node_ij(g.Nx / 2, g.Ny, magic, i, j)) return;
     i *= 2;
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    cls = pdl_fresh(cls);
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     float x[19], y[19];
@@ -379,11 +385,13 @@ inline bool pairs_fit(const Grid3 &g, const void *fo, const void *fi, const void
 template <bool CLS>
 void launch_trt2(float *fo, const float *fi, float *rho, float *ux, float *uy, float *uz,
                  const uint8_t *cls, const Grid3 &g, float sp, float sm, cudaStream_t s) {
-    if (offsets_fit_int(g, 19))
-        fused_trt2_k<CLS, int><<<pair_grid(g), BX, 0, s>>>(fo, fi, rho, ux, uy, uz, cls, g, pair_magic(g), sp, sm);
+    const auto k = offsets_fit_int(g, 19) ? fused_trt2_k<CLS, int> : fused_trt2_k<CLS, long long>;
+    const unsigned m = pair_magic(g);
+    // beside the cut-node kernel the launch follows an event wait: a plain one
+    if (CLS)
+        k<<<pair_grid(g), BX, 0, s>>>(fo, fi, rho, ux, uy, uz, cls, g, m, sp, sm);
     else
-        fused_trt2_k<CLS, long long><<<pair_grid(g), BX, 0, s>>>(fo, fi, rho, ux, uy, uz, cls, g,
-                                                                 pair_magic(g), sp, sm);
+        launch_pdl(k, pair_grid(g), dim3(BX), s, fo, fi, rho, ux, uy, uz, cls, g, m, sp, sm);
 }
 
 // The cut nodes (class 2) of a compact table, one thread per record.
@@ -834,6 +842,9 @@ __global__ void __launch_bounds__(BX) cavity_step_k(T *__restrict__ fo, const T 
                                                      const uint8_t *__restrict__ solid, Grid3 g,
                                                      T omega, T u_lid) {
     NODE3_IJK
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     T p[19];
@@ -871,6 +882,9 @@ __global__ void __launch_bounds__(BX) cavity_step2_k(float *__restrict__ fo, con
     const int k = blockIdx.z;
     if (!node_ij(g.Nx / 2, g.Ny, magic, i, j)) return;
     i *= 2;
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    solid = pdl_fresh(solid);
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     float x[19], y[19];
@@ -920,6 +934,9 @@ __global__ void __launch_bounds__(BX, 3) natconv_step_k(T *__restrict__ fo, cons
                                                       Grid3 g, T w_f, T w_T, T beta_g, T T_ref,
                                                       T T_hot, T T_cold) {
     NODE3_IJK
+    pdl_wait();
+    fi = pdl_fresh(fi);
+    gi = pdl_fresh(gi);
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
     const I P = (I)g.plane;
     const Pull3<I> s = pull_geometry<I>(g, i, j, k);
@@ -1114,19 +1131,19 @@ int kb_cavity_step_3d(void *f_out, const void *f_in, void *rho, void *ux, void *
     cudaStream_t s = kb::as_stream(stream);
     if (dtype == KB_F32 && pairs_fit(g, f_out, f_in, rho, ux, uy, uz, is_solid)) {
         const auto k2 = offsets_fit_int(g, 19) ? cavity_step2_k<int> : cavity_step2_k<long long>;
-        k2<<<pair_grid(g), BX, 0, s>>>((float *)f_out, (const float *)f_in, (float *)rho, (float *)ux,
-                                       (float *)uy, (float *)uz, is_solid, g, pair_magic(g), (float)omega,
-                                       (float)u_lid);
+        kb::launch_pdl(k2, pair_grid(g), dim3(BX), s, (float *)f_out, (const float *)f_in, (float *)rho,
+                       (float *)ux, (float *)uy, (float *)uz, is_solid, g, pair_magic(g), (float)omega,
+                       (float)u_lid);
         return kb::check_launch(what);
     }
     KB3_DISPATCH_PLAIN(what, dtype,
         if (offsets_fit_int(g, 19))
-            (cavity_step_k<T, int><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
-                (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
+            (kb::launch_pdl(cavity_step_k<T, int>, node_grid(grid3(Nx, Ny, Nz)), dim3(BX), s,
+            (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
                 (T)u_lid));
         else
-            (cavity_step_k<T, long long><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
-                (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
+            (kb::launch_pdl(cavity_step_k<T, long long>, node_grid(grid3(Nx, Ny, Nz)), dim3(BX), s,
+            (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, (T *)uz, is_solid, g, (T)omega,
                 (T)u_lid)));
 }
 
@@ -1142,12 +1159,12 @@ int kb_natconv_step_3d(void *f_out, const void *f_in, void *g_out, const void *g
     cudaStream_t s = kb::as_stream(stream);
     KB3_DISPATCH_PLAIN(what, dtype,
         if (offsets_fit_int(g, 19))
-            (natconv_step_k<T, int><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
-                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
+            (kb::launch_pdl(natconv_step_k<T, int>, node_grid(grid3(Nx, Ny, Nz)), dim3(BX), s,
+            (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
                 (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold));
         else
-            (natconv_step_k<T, long long><<<node_grid(grid3(Nx, Ny, Nz)), BX, 0, s>>>(
-                (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
+            (kb::launch_pdl(natconv_step_k<T, long long>, node_grid(grid3(Nx, Ny, Nz)), dim3(BX), s,
+            (T *)f_out, (const T *)f_in, (T *)g_out, (const T *)g_in, g, (T)omega_f, (T)omega_T,
                 (T)beta_g, (T)T_ref, (T)T_hot, (T)T_cold)));
 }
 
@@ -1179,24 +1196,24 @@ int trt3d_step(const char *what, void *f_out, const void *f_in, void *rho, void 
     const dim3 grid = node_grid(g);
     if (dtype == KB_F64) {
         if (i32)
-            fused_trt_k<double, int><<<grid, BX, 0, s>>>(
-                (double *)f_out, (const double *)f_in, (double *)rho, (double *)ux, (double *)uy,
+            kb::launch_pdl(fused_trt_k<double, int>, grid, dim3(BX), s,
+            (double *)f_out, (const double *)f_in, (double *)rho, (double *)ux, (double *)uy,
                 (double *)uz, is_solid, g, sp, sm);
         else
-            fused_trt_k<double, long long><<<grid, BX, 0, s>>>(
-                (double *)f_out, (const double *)f_in, (double *)rho, (double *)ux, (double *)uy,
+            kb::launch_pdl(fused_trt_k<double, long long>, grid, dim3(BX), s,
+            (double *)f_out, (const double *)f_in, (double *)rho, (double *)ux, (double *)uy,
                 (double *)uz, is_solid, g, sp, sm);
     } else if (dtype == KB_F32) {
         if (pairs_fit(g, f_out, f_in, rho, ux, uy, uz, is_solid))
             launch_trt2<false>((float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
                                (float *)uz, is_solid, g, (float)sp, (float)sm, s);
         else if (i32)
-            fused_trt_k<float, int><<<grid, BX, 0, s>>>(
-                (float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
+            kb::launch_pdl(fused_trt_k<float, int>, grid, dim3(BX), s,
+            (float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
                 (float *)uz, is_solid, g, (float)sp, (float)sm);
         else
-            fused_trt_k<float, long long><<<grid, BX, 0, s>>>(
-                (float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
+            kb::launch_pdl(fused_trt_k<float, long long>, grid, dim3(BX), s,
+            (float *)f_out, (const float *)f_in, (float *)rho, (float *)ux, (float *)uy,
                 (float *)uz, is_solid, g, (float)sp, (float)sm);
     } else if (dtype == KB_F32_DEV || dtype == KB_F16_DEV || dtype == KB_BF16_DEV ||
                dtype == KB_F16_DEV_SR || dtype == KB_BF16_DEV_SR) {
