@@ -12,8 +12,11 @@
 //
 // Schedule: the nodes of all active cases are cut into tiles of `tile_nodes`
 // consecutive nodes of one case.  The kernel is launched cooperatively with
-// blocks_per_sm x SMs blocks; each step the blocks stride over the active
-// tile list, then meet at a grid barrier (spin bounded by an iteration
+// blocks_per_sm x SMs blocks; each step the blocks share the active tile list
+// (untuned: equal runs of consecutive 256-node tiles, which balances to one
+// tile and keeps a block in one case: 48 cavities of 64^2 to 512^2 in FP16 ran
+// at 106 GLUPS against 64 with every nblocks-th tile; tuned or given a tile
+// size: every nblocks-th tile), then meet at a grid barrier (spin bounded by an iteration
 // limit; a timeout sets an error flag that every block sees and returns on).
 // Every `check_every` steps the residual of each case is reduced on the device
 // (FP64 atomics per tile), block 0 retires converged / finished / non-finite
@@ -110,6 +113,61 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return t;
 }
 
+// MRT collision on deviations, in place, for one node (V = float) or two
+// (float2): collide_mrt_2d_kernel! (collide_mrt_2d.jl:54-106) with s_e = s_eps
+// = 1.4, s_q = 1.2 multiplied out.  With a = d1..d4, g = d5..d8 sums, R = 3 rho
+// |u|^2 = 3 (jx ux + jy uy) and the relaxed moments substituted,
+//   (c9 drho - c36 es - c18 eps)  = (5.6 (d0 + g) + 2 a + 1.4 R) / 36   = A
+//   (c9 drho + c18 es + c36 eps)  = (1.4 (d0 + a) - 2.2 g + 1.4 R) / 36 = D
+//   c6 (jx - qx*) = 0.3 (d1 - d3) + 0.4 X,   X = d5 - d6 - d7 + d8      = ax
+// and likewise in y.  The rest population and the diagonal momentum parts
+// come from conservation, drho - 4 (A + D) and (jx - 2 ax) / 4, so neither
+// mass nor momentum drifts with the rounding of the coefficients.  About 65
+// operations; moment by moment it was about 130, and the sweep was bound by
+// them.
+__device__ __forceinline__ float inv_rho(float a) { return 1.0f / a; }
+__device__ __forceinline__ float2 inv_rho(float2 a) { return vrcp_fast(a); }
+
+template <typename V>
+__device__ __forceinline__ void mrt_collide(V *d, float s_nu, V &ux, V &uy) {
+    const auto K = [](float x) { return vsplat(x, V()); };
+    const V a1 = vadd(d[1], d[3]), a2 = vadd(d[2], d[4]);
+    const V t13 = vsub(d[1], d[3]), t24 = vsub(d[2], d[4]);
+    const V s57 = vadd(d[5], d[7]), s68 = vadd(d[6], d[8]);
+    const V m57 = vsub(d[5], d[7]), m68 = vsub(d[6], d[8]);
+    const V da = vadd(a1, a2), dg = vadd(s57, s68);
+    const V d0a = vadd(d[0], da), d0g = vadd(d[0], dg);
+    const V drho = vadd(d0a, dg);
+    const V X = vsub(m57, m68), Y = vadd(m57, m68);
+    const V jx = vadd(t13, X), jy = vadd(t24, Y);
+    const V inv = inv_rho(vadd(K(1.0f), drho));
+    ux = vmul(jx, inv);
+    uy = vmul(jy, inv);
+    const V exx = vmul(jx, ux), eyy = vmul(jy, uy);
+    const V cR = vmul(K(4.2f / 36.0f), vadd(exx, eyy));
+    const V A = vfma(K(5.6f / 36.0f), d0g, vfma(K(2.0f / 36.0f), da, cR));
+    const V D = vfma(K(1.4f / 36.0f), d0a, vfma(K(-2.2f / 36.0f), dg, cR));
+    // 1/4 of the relaxed second-order moments
+    const float s4 = 0.25f * s_nu, o4 = 0.25f - s4;
+    const V p4 = vfma(K(s4), vsub(exx, eyy), vmul(K(o4), vsub(a1, a2)));
+    const V x4 = vfma(K(s4), vmul(jx, uy), vmul(K(o4), vsub(s57, s68)));
+    const V ax = vfma(K(0.3f), t13, vmul(K(0.4f), X));
+    const V ay = vfma(K(0.3f), t24, vmul(K(0.4f), Y));
+    const V bx = vfma(K(-0.5f), ax, vmul(K(0.25f), jx));
+    const V by = vfma(K(-0.5f), ay, vmul(K(0.25f), jy));
+    const V Ap = vadd(A, p4), Am = vsub(A, p4), Dp = vadd(D, x4), Dm = vsub(D, x4);
+    const V bs = vadd(bx, by), bd = vsub(bx, by);
+    d[0] = vfma(K(-4.0f), vadd(A, D), drho);
+    d[1] = vadd(Ap, ax);
+    d[3] = vsub(Ap, ax);
+    d[2] = vadd(Am, ay);
+    d[4] = vsub(Am, ay);
+    d[5] = vadd(Dp, bs);
+    d[7] = vsub(Dp, bs);
+    d[8] = vadd(Dm, bd);
+    d[6] = vsub(Dm, bd);
+}
+
 // One node of one case: pull (half-way bounce-back), Zou-He lid on the top
 // row, MRT on deviations; returns the pre-collision velocity.
 template <typename R, bool SR>
@@ -138,46 +196,8 @@ __device__ __forceinline__ void node_update(const R *__restrict__ src, R *__rest
         d[8] = d[6] - h + m;
         d[7] = d[5] + h - m;
     }
-    // moments of the deviations (rows of M, collide_mrt_2d.jl:17-28)
-    const float drho = d[0] + d[1] + d[2] + d[3] + d[4] + d[5] + d[6] + d[7] + d[8];
-    const float dg = d[5] + d[6] + d[7] + d[8];
-    const float da = d[1] + d[2] + d[3] + d[4];
-    const float e_d = -4.0f * d[0] - da + 2.0f * dg;
-    const float eps_d = 4.0f * d[0] - 2.0f * da + dg;
-    const float jx = d[1] - d[3] + d[5] - d[6] - d[7] + d[8];
-    const float qx = -2.0f * (d[1] - d[3]) + d[5] - d[6] - d[7] + d[8];
-    const float jy = d[2] - d[4] + d[5] + d[6] - d[7] - d[8];
-    const float qy = -2.0f * (d[2] - d[4]) + d[5] + d[6] - d[7] - d[8];
-    const float pxx = d[1] - d[2] + d[3] - d[4];
-    const float pxy = d[5] - d[6] + d[7] - d[8];
-    const float rho = 1.0f + drho;
-    const float inv = 1.0f / rho;
-    ux = jx * inv;
-    uy = jy * inv;
-    const float r3u = 3.0f * rho * (ux * ux + uy * uy);
-    const float s_e = 1.4f, s_eps = 1.4f, s_q = 1.2f;
-    // post-collision deviation moments: m*_d = m_d - S (m - m_eq)
-    const float es = e_d - s_e * (e_d + 2.0f * drho - r3u);
-    const float ep = eps_d - s_eps * (eps_d - drho + r3u);
-    const float qxs = qx - s_q * (qx + jx);
-    const float qys = qy - s_q * (qy + jy);
-    const float ps = pxx - s_nu * (pxx - rho * (ux * ux - uy * uy));
-    const float pxys = pxy - s_nu * (pxy - rho * ux * uy);
-    const float r = drho;
-    const float c9 = 1.0f / 9.0f, c36 = 1.0f / 36.0f, c18 = 1.0f / 18.0f, c6 = 1.0f / 6.0f,
-                c4 = 0.25f, c12 = 1.0f / 12.0f;
-    const float base_a = c9 * r - c36 * es - c18 * ep;
-    const float base_d = c9 * r + c18 * es + c36 * ep;
-    float o[9];
-    o[0] = c9 * r - c9 * es + c9 * ep;
-    o[1] = base_a + c6 * jx - c6 * qxs + c4 * ps;
-    o[2] = base_a + c6 * jy - c6 * qys - c4 * ps;
-    o[3] = base_a - c6 * jx + c6 * qxs + c4 * ps;
-    o[4] = base_a - c6 * jy + c6 * qys - c4 * ps;
-    o[5] = base_d + c6 * jx + c12 * qxs + c6 * jy + c12 * qys + c4 * pxys;
-    o[6] = base_d - c6 * jx - c12 * qxs + c6 * jy + c12 * qys - c4 * pxys;
-    o[7] = base_d - c6 * jx - c12 * qxs - c6 * jy - c12 * qys + c4 * pxys;
-    o[8] = base_d + c6 * jx + c12 * qxs - c6 * jy - c12 * qys - c4 * pxys;
+    mrt_collide(d, s_nu, ux, uy);
+    const float *o = d;
     if (SR) {
         // stochastic rounding: populations (0,1), (2,3), (4,5), (6,7), (8,-)
         // share one cvt.rs and one 32-bit random word
@@ -287,50 +307,8 @@ __device__ __forceinline__ void pair_finish(float2 *d, R *__restrict__ dst, int 
         d[8] = vadd(vsub(d[6], h), m);
         d[7] = vsub(vadd(d[5], h), m);
     }
-    const float2 drho = vadd(vadd(vadd(d[0], d[1]), vadd(d[2], d[3])),
-                             vadd(vadd(d[4], d[5]), vadd(vadd(d[6], d[7]), d[8])));
-    const float2 dg = vadd(vadd(d[5], d[6]), vadd(d[7], d[8]));
-    const float2 da = vadd(vadd(d[1], d[2]), vadd(d[3], d[4]));
-    const float2 e_d = vadd(vsub(vmul(vsplat(-4.0f, z), d[0]), da), vmul(vsplat(2.0f, z), dg));
-    const float2 eps_d = vadd(vsub(vmul(vsplat(4.0f, z), d[0]), vmul(vsplat(2.0f, z), da)), dg);
-    const float2 t13 = vsub(d[1], d[3]), t24 = vsub(d[2], d[4]);
-    const float2 jx = vadd(t13, vsub(vsub(vadd(d[5], d[8]), d[6]), d[7]));
-    const float2 qx = vadd(vmul(vsplat(-2.0f, z), t13), vsub(vsub(vadd(d[5], d[8]), d[6]), d[7]));
-    const float2 jy = vadd(t24, vsub(vsub(vadd(d[5], d[6]), d[7]), d[8]));
-    const float2 qy = vadd(vmul(vsplat(-2.0f, z), t24), vsub(vsub(vadd(d[5], d[6]), d[7]), d[8]));
-    const float2 pxx = vsub(vadd(d[1], d[3]), vadd(d[2], d[4]));
-    const float2 pxy = vsub(vadd(d[5], d[7]), vadd(d[6], d[8]));
-    const float2 rho = vadd(vsplat(1.0f, z), drho);
-    const float2 inv = vrcp_fast(rho);
-    ux = vmul(jx, inv);
-    uy = vmul(jy, inv);
-    const float2 r3u = vmul(vmul(vsplat(3.0f, z), rho), vfma(ux, ux, vmul(uy, uy)));
-    const float s_e = 1.4f, s_eps = 1.4f, s_q = 1.2f;
-    const float2 es = vsub(e_d, vmul(vsplat(s_e, z), vsub(vadd(e_d, vmul(vsplat(2.0f, z), drho)), r3u)));
-    const float2 ep = vsub(eps_d, vmul(vsplat(s_eps, z), vadd(vsub(eps_d, drho), r3u)));
-    const float2 qxs = vsub(qx, vmul(vsplat(s_q, z), vadd(qx, jx)));
-    const float2 qys = vsub(qy, vmul(vsplat(s_q, z), vadd(qy, jy)));
-    const float2 ps = vsub(pxx, vmul(vsplat(s_nu, z), vsub(pxx, vmul(rho, vsub(vmul(ux, ux), vmul(uy, uy))))));
-    const float2 pxys = vsub(pxy, vmul(vsplat(s_nu, z), vsub(pxy, vmul(rho, vmul(ux, uy)))));
-    const float c9 = 1.0f / 9.0f, c36 = 1.0f / 36.0f, c18 = 1.0f / 18.0f, c6 = 1.0f / 6.0f,
-                c4 = 0.25f, c12 = 1.0f / 12.0f;
-    const float2 base_a = vsub(vsub(vmul(vsplat(c9, z), drho), vmul(vsplat(c36, z), es)), vmul(vsplat(c18, z), ep));
-    const float2 base_d = vadd(vadd(vmul(vsplat(c9, z), drho), vmul(vsplat(c18, z), es)), vmul(vsplat(c36, z), ep));
-    const float2 ax = vsub(vmul(vsplat(c6, z), jx), vmul(vsplat(c6, z), qxs));   // c6 jx - c6 qx*
-    const float2 ay = vsub(vmul(vsplat(c6, z), jy), vmul(vsplat(c6, z), qys));
-    const float2 bx = vadd(vmul(vsplat(c6, z), jx), vmul(vsplat(c12, z), qxs));  // c6 jx + c12 qx*
-    const float2 by = vadd(vmul(vsplat(c6, z), jy), vmul(vsplat(c12, z), qys));
-    const float2 p4 = vmul(vsplat(c4, z), ps), x4 = vmul(vsplat(c4, z), pxys);
-    float2 o[9];
-    o[0] = vmul(vsplat(c9, z), vadd(vsub(drho, es), ep));
-    o[1] = vadd(vadd(base_a, ax), p4);
-    o[2] = vsub(vadd(base_a, ay), p4);
-    o[3] = vadd(vsub(base_a, ax), p4);
-    o[4] = vsub(vsub(base_a, ay), p4);
-    o[5] = vadd(vadd(vadd(base_d, bx), by), x4);
-    o[6] = vsub(vadd(vsub(base_d, bx), by), x4);
-    o[7] = vadd(vsub(vsub(base_d, bx), by), x4);
-    o[8] = vsub(vsub(vadd(base_d, bx), by), x4);
+    mrt_collide(d, s_nu, ux, uy);
+    const float2 *o = d;
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
         if (SR) {
@@ -344,7 +322,7 @@ __device__ __forceinline__ void pair_finish(float2 *d, R *__restrict__ dst, int 
 
 template <typename R, bool SR>
 __global__ void __launch_bounds__(BT, KB_BATCH_MIN_BLOCKS) batch_k(BatchState D, int n_cases, int n_tiles_all, int tile_nodes,
-                                               int max_steps, int check_every, float tol,
+                                               int ranges, int max_steps, int check_every, float tol,
                                                long long spin_limit, uint32_t seed) {
     __shared__ double sh[BT / 32];
     const unsigned nblocks = gridDim.x;
@@ -355,11 +333,18 @@ __global__ void __launch_bounds__(BT, KB_BATCH_MIN_BLOCKS) batch_k(BatchState D,
         R *dst = (R *)((s & 1) ? D.pool_a : D.pool_b);
         const bool check = (s + 1) % check_every == 0;
         const bool save = (s + 2) % check_every == 0;
-        for (int t = blockIdx.x; t < nt; t += nblocks) {
+        // ranges: this block's share of the list is one run of tiles, taken a
+        // case at a time as one range of nodes (the list is in node order and
+        // drops whole cases); otherwise every nblocks-th tile
+        const int t1 = ranges ? (int)((long long)nt * (blockIdx.x + 1) / nblocks) : nt;
+        for (int t = ranges ? (int)((long long)nt * blockIdx.x / nblocks) : blockIdx.x; t < t1;) {
             const Tile T = D.tiles[t];
             const CaseDesc C = D.cases[T.c];
             const int NN = C.N * C.N;
-            const int end = min(T.start + tile_nodes, NN);
+            int take = 1;
+            if (ranges) take = min((NN - T.start + tile_nodes - 1) / tile_nodes, t1 - t);
+            const int end = min(T.start + take * tile_nodes, NN);
+            t += ranges ? take : (int)nblocks;
             double du2 = 0.0, u2 = 0.0;
             if (C.N & 1) {
                 // odd N: rows start at odd offsets, so one node per thread
@@ -573,7 +558,7 @@ int reset(kb_batch *b, cudaStream_t s) {
 }
 
 template <typename R, bool SR = false>
-int launch(kb_batch *b, int max_steps, int check_every, double tol, int blocks_per_sm,
+int launch(kb_batch *b, int max_steps, int check_every, double tol, int blocks_per_sm, bool ranges,
            cudaStream_t s) {
     const ScalLayout L = scal_layout(b->n_cases);
     BatchState D;
@@ -600,7 +585,8 @@ int launch(kb_batch *b, int max_steps, int check_every, double tol, int blocks_p
     // seconds is declared timed out
     long long spin = 1ll << 24;
     uint32_t seed = b->runs++;  // fresh random bits for every run of the batch
-    void *args[] = {&D, &n_cases, &n_all, &tn, &max_steps, &check_every, &tolf, &spin, &seed};
+    int rng = ranges ? 1 : 0;
+    void *args[] = {&D, &n_cases, &n_all, &tn, &rng, &max_steps, &check_every, &tolf, &spin, &seed};
     dim3 grid(bpsm * kb::sm_count()), block(BT);
     e = cudaLaunchCooperativeKernel((void *)batch_k<R, SR>, grid, block, args, 0, s);
     if (e != cudaSuccess) return cuda_err("kb_batch_run: cooperative launch", e);
@@ -704,6 +690,7 @@ int kb_batch_run(kb_batch *b, int max_steps, int check_every, double tol, int ti
     KB_REQUIRE(check_every >= 2, "kb_batch_run: check_every must be >= 2");
     KB_REQUIRE(max_steps >= check_every && max_steps % check_every == 0,
                "kb_batch_run: max_steps must be a positive multiple of check_every");
+    const bool ranges = tile_nodes <= 0 && b->tuned_tile <= 0;
     if (tile_nodes <= 0) tile_nodes = b->tuned_tile > 0 ? b->tuned_tile : 256;
     if (blocks_per_sm <= 0) blocks_per_sm = b->tuned_bpsm > 0 ? b->tuned_bpsm : 0;
     KB_REQUIRE(tile_nodes % 32 == 0 && tile_nodes <= (1 << 20),
@@ -714,12 +701,12 @@ int kb_batch_run(kb_batch *b, int max_steps, int check_every, double tol, int ti
         if (int r = reset(b, s)) return r;
     }
     switch (b->dtype) {
-        case KB_F16_DEV: return launch<__half>(b, max_steps, check_every, tol, blocks_per_sm, s);
-        case KB_BF16_DEV: return launch<__nv_bfloat16>(b, max_steps, check_every, tol, blocks_per_sm, s);
-        case KB_F16_DEV_SR: return launch<__half, true>(b, max_steps, check_every, tol, blocks_per_sm, s);
+        case KB_F16_DEV: return launch<__half>(b, max_steps, check_every, tol, blocks_per_sm, ranges, s);
+        case KB_BF16_DEV: return launch<__nv_bfloat16>(b, max_steps, check_every, tol, blocks_per_sm, ranges, s);
+        case KB_F16_DEV_SR: return launch<__half, true>(b, max_steps, check_every, tol, blocks_per_sm, ranges, s);
         case KB_BF16_DEV_SR:
-            return launch<__nv_bfloat16, true>(b, max_steps, check_every, tol, blocks_per_sm, s);
-        default: return launch<float>(b, max_steps, check_every, tol, blocks_per_sm, s);
+            return launch<__nv_bfloat16, true>(b, max_steps, check_every, tol, blocks_per_sm, ranges, s);
+        default: return launch<float>(b, max_steps, check_every, tol, blocks_per_sm, ranges, s);
     }
 }
 
@@ -772,9 +759,9 @@ int kb_batch_autotune(kb_batch *b, int trial_steps, int *best_tile, int *best_bp
     KB_REQUIRE(b, "kb_batch_autotune: null handle");
     KB_REQUIRE(trial_steps >= 2 && trial_steps % 2 == 0, "kb_batch_autotune: trial_steps must be even and >= 2");
     cudaStream_t s = kb::as_stream(stream);
-    // the candidates: tile sizes x every residency up to the occupancy limit;
-    // the fixed schedule is what kb_batch_run takes untuned (256-node tiles,
-    // as many blocks per SM as fit)
+    // the candidates: tile sizes x every residency up to the occupancy limit
+    // (the fixed schedule they are compared with: 256-node tiles, as many
+    // blocks per SM as fit), and the untuned schedule
     const int occ = batch_occupancy(b->dtype);
     if (occ < 1) return kb::set_error(KB_ERR_UNSUPPORTED, "kb_batch_autotune: kernel does not fit an SM");
     const int tiles[] = {256, 512, 1024, 2048, 4096};
@@ -801,10 +788,29 @@ int kb_batch_autotune(kb_batch *b, int trial_steps, int *best_tile, int *best_bp
             if (tn == 256 && bp == occ) fixed = mlups;
             if (mlups > best) { best = mlups; bt = tn; bb = bp; }
         }
+    // the untuned schedule (ranges of the 256-node list at the occupancy limit)
+    bool ranges = false;
+    {
+        b->tuned_tile = b->tuned_bpsm = 0;
+        if (int r = build_tiles(b, 256)) return r;
+        if (int r = reset(b, s)) return r;
+        cudaEventRecord(e0, s);
+        if (int r = kb_batch_run(b, trial_steps, trial_steps, 0.0, 0, 0, stream)) return r;
+        cudaEventRecord(e1, s);
+        cudaError_t e = cudaEventSynchronize(e1);
+        if (e != cudaSuccess) return cuda_err("kb_batch_autotune", e);
+        long long up = 0;
+        int live = 0, tout = 0;
+        if (int r = kb_batch_status(b, &up, &live, &tout, stream)) return r;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        const double mlups = (double)up / (ms * 1e-3) / 1e6;
+        if (mlups > best) { best = mlups; bt = 256; bb = occ; ranges = true; }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    b->tuned_tile = bt;
-    b->tuned_bpsm = bb;
+    b->tuned_tile = ranges ? 0 : bt;
+    b->tuned_bpsm = ranges ? 0 : bb;
     if (int r = build_tiles(b, bt)) return r;
     if (int r = reset(b, s)) return r;
     if (best_tile) *best_tile = bt;
