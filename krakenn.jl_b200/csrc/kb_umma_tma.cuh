@@ -7,13 +7,17 @@
 // whatever N is, so an N = 32 tile reaches 1/8 of the tensor rate from one
 // issuer; several CTAs per SM, each with its own ring, MMA lane and share of
 // TMEM, multiply the issue rate.  In each CTA:
-//   warp 0    producer: lane 0 waits for a free ring stage (`empty`), posts
-//             the stage's byte count on its `full` barrier and issues the
-//             step's cp.async.bulk.tensor copies, one per operand box;
-//   warp 1    MMA: allocates TMEM (two accumulators of the tile width);
-//             lane 0 waits `full`, issues the step's tcgen05.mma, commits to
-//             the stage's `empty` barrier, and to `acc_full` after a tile's
-//             last step;
+//   warp 0    producer: waits for a free ring stage (`empty`), posts the
+//             stage's byte count on its `full` barrier and issues the step's
+//             cp.async.bulk.tensor copies, one per operand box;
+//   warp 1    MMA: allocates TMEM (two accumulators of the tile width), waits
+//             `full`, issues the step's tcgen05.mma, commits to the stage's
+//             `empty` barrier, and to `acc_full` after a tile's last step.
+//             Both warps run their loops converged and one elected lane
+//             issues: descriptors and coordinates then stay warp-uniform, and
+//             descriptor steps are one add to the low word (Desc).  With the
+//             loops on lane 0 alone a batch-16 256^2 gradient took 2645 us,
+//             with an elected lane 2491, with the stepped descriptors 2482;
 //   warps 2.. epilogue, TM_EPI warps per TMEM lane quarter: warp w reads
 //             TMEM lanes 32(w%4)..+31 (tile rows) of the finished
 //             accumulator, every TM_EPI-th group of 8 columns, calls op.store
@@ -67,12 +71,47 @@ __device__ __forceinline__ uint64_t sdesc_sw(uint32_t saddr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (layout << 61);
 }
 
-// Descriptor of MMA kk (16 K elements) of a stage's operand tile.
-__device__ __forceinline__ uint64_t op_desc(uint32_t base, bool mn, uint32_t swz, int kk) {
-    return mn ? sdesc_sw(base + (uint32_t)kk * 16u * swz, 64u * swz, 8u * swz, swz)
-              : sdesc_sw(base + (uint32_t)kk * 32u, 16u, 8u * swz, swz);
+// A descriptor as two words.  Operand tiles lie below 256 KB of shared memory,
+// so stepping the start address is an add to the low word that never carries
+// out of its 14 address bits; the high word (strides, swizzle) stays put.
+struct Desc { uint32_t lo, hi; };
+__device__ __forceinline__ Desc desc_sw(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t swz) {
+    const uint64_t d = sdesc_sw(saddr, lbo, sbo, swz);
+    return Desc{(uint32_t)d, (uint32_t)(d >> 32)};
+}
+// K-major tile (MMA kk starts 32 bytes = 2 units further) and MN-major tile
+// (16 rows of `swz` bytes = swz units further).
+__device__ __forceinline__ Desc desc_k(uint32_t base, uint32_t swz) { return desc_sw(base, 16u, 8u * swz, swz); }
+__device__ __forceinline__ Desc desc_mn(uint32_t base, uint32_t swz) { return desc_sw(base, 64u * swz, 8u * swz, swz); }
+
+__device__ __forceinline__ void mma_at(uint32_t tmem_d, const Desc &a, uint32_t da, const Desc &b, uint32_t db,
+                                       uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t"
+        "mov.b64 x, {%1, %2};\n\tmov.b64 y, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n\t}"
+        ::"r"(tmem_d), "r"(a.lo + da), "r"(a.hi), "r"(b.lo + db), "r"(b.hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// N MMAs along K of one operand pair, `sa` / `sb` descriptor units apart.
+template <int N>
+__device__ __forceinline__ void mma_run(uint32_t acc, const Desc &a, uint32_t da, uint32_t sa, const Desc &b,
+                                        uint32_t db, uint32_t sb, uint32_t idesc, uint32_t accumulate) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+        mma_at(acc, a, da + (uint32_t)k * sa, b, db + (uint32_t)k * sb, idesc, k ? 1u : accumulate);
 }
 
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// mbar_wait by a converged warp: every lane has seen the phase complete.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, long long limit) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
 __device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
@@ -162,7 +201,7 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
     uint64_t *acc_full = empty + nstages, *acc_empty = acc_full + 2, *drain = acc_empty + 2;
     uint64_t *resbar = drain + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(resbar + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t cols = op.acc_cols;
     const int nbuf = op.nbuf;
     const int ntiles = (int)(tiles.x * tiles.y * tiles.z);  // < 2^31 (checked by launch_tma)
@@ -188,7 +227,7 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
 
     // Ring position (slot s, parity `par` of its current use) and tile
@@ -196,9 +235,9 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
     // single threads, and a division per step would be their critical path.
     if (warp == 0) {
         // ---------------------------------------------------------- producer
-        if (lane == 0) {
-            op.prefetch();
-            if (op.res_bytes) {
+        {
+            if (elect_one()) op.prefetch();
+            if (op.res_bytes && elect_one()) {
                 expect_tx(smem_u32(resbar), op.res_bytes);
                 op.issue_res(res, smem_u32(resbar));
             }
@@ -213,11 +252,12 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
                 const uint32_t tx = op.step_tx(t);
                 typename Op::Cursor cur = op.begin(t, k0);
                 for (int kt = k0; kt < k1; ++kt, ++g) {
-                    if (g >= nstages && !(ok = mbar_wait(&empty[s], par ^ 1u, spin))) break;
+                    if (g >= nstages && !(ok = mbar_wait_warp(&empty[s], par ^ 1u, spin))) break;
                     const uint32_t sa = base + (uint32_t)s * stage_bytes;
                     const uint32_t bar = smem_u32(&full[s]);
-                    expect_tx(bar, tx);
-                    op.issue(cur, t, sa, sa + op.a_bytes, bar);
+                    const bool lead = elect_one();
+                    if (lead) expect_tx(bar, tx);
+                    op.issue(cur, t, sa, sa + op.a_bytes, bar, lead);
                     if (++s == nstages) {
                         s = 0;
                         par ^= 1u;
@@ -232,44 +272,47 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
                     par ^= 1u;
                 }
                 --s;
-                if (!mbar_wait(&full[s], par, spin)) ok = false;
+                if (!mbar_wait_warp(&full[s], par, spin)) ok = false;
             }
-            if (op.res_bytes && !mbar_wait(resbar, 0u, spin)) ok = false;
+            if (op.res_bytes && !mbar_wait_warp(resbar, 0u, spin)) ok = false;
         }
         __syncwarp();
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
-        if (lane == 0) {
+        {
             const uint32_t idesc = idesc_bf16(op.bn, Op::A_MN, Op::B_MN);
             int s = 0, j = 0;
             uint32_t par = 0;
-            if (op.res_bytes) ok = mbar_wait(resbar, 0u, spin);
+            if (op.res_bytes) ok = mbar_wait_warp(resbar, 0u, spin);
             TileCursor tc(tiles);
             for (int T = blockIdx.x; T < ntiles && ok; T += gridDim.x, ++j) {
                 const int buf = nbuf == 2 ? (j & 1) : 0, use = nbuf == 2 ? (j >> 1) : j;
-                if (use >= 1 && !(ok = mbar_wait(&acc_empty[buf], (uint32_t)((use - 1) & 1), spin))) break;
+                if (use >= 1 && !(ok = mbar_wait_warp(&acc_empty[buf], (uint32_t)((use - 1) & 1), spin))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint3 t = tc.at(T);
                 int k0, k1;
                 op.k_range(t, k0, k1);
                 const uint32_t acc = tmem + (uint32_t)buf * cols;
                 for (int kt = k0; kt < k1; ++kt) {
-                    if (!(ok = mbar_wait(&full[s], par, spin))) break;
+                    if (!(ok = mbar_wait_warp(&full[s], par, spin))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = base + (uint32_t)s * stage_bytes;
-                    op.mma(acc, sa, sa + op.a_bytes, res, kt, k0, t, idesc);
-                    mma_commit(&empty[s]);
+                    if (elect_one()) {
+                        op.mma(acc, sa, sa + op.a_bytes, res, kt, k0, t, idesc);
+                        mma_commit(&empty[s]);
+                    }
+                    __syncwarp();
                     if (++s == nstages) {
                         s = 0;
                         par ^= 1u;
                     }
                 }
                 if (!ok) break;
-                mma_commit(&acc_full[buf]);
+                if (elect_one()) mma_commit(&acc_full[buf]);
             }
             // every MMA issued above is complete once this commit arrives
-            mma_commit(drain);
-            if (!mbar_wait(drain, 0u, spin)) ok = false;
+            if (elect_one()) mma_commit(drain);
+            if (!mbar_wait_warp(drain, 0u, spin)) ok = false;
         }
         __syncwarp();
     } else {
@@ -371,10 +414,9 @@ struct ConvTma : ConvStore, TmaBase {
         u.wk = 0;
         return u;
     }
-    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar) const {
-        if (u.c < c1) tma4(sa, &x1, u.c, u.x + u.dx, u.y + u.dy, u.b, bar);
-        else tma4(sa, &x2, u.c - c1, u.x + u.dx, u.y + u.dy, u.b, bar);
-        tma2(sb, &w, u.wk, (int)t.y * bn, bar);
+    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
+        if (lead) { if (u.c < c1) tma4(sa, &x1, u.c, u.x + u.dx, u.y + u.dy, u.b, bar); else tma4(sa, &x2, u.c - c1, u.x + u.dx, u.y + u.dy, u.b, bar); }
+        if (lead) tma2(sb, &w, u.wk, (int)t.y * bn, bar);
         u.wk += e;
         u.c += e;
         if (u.c == C) {
@@ -388,11 +430,11 @@ struct ConvTma : ConvStore, TmaBase {
     __device__ void issue_res(uint32_t, uint32_t) const {}
     __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int k0, const uint3 &,
                         uint32_t idesc) const {
-        const bool first = kt == k0;
-        const uint32_t s = 2u * (uint32_t)e;
-        for (int kk = 0; kk < e / 16; ++kk)
-            mma_bf16(acc, op_desc(sa, false, s, kk), op_desc(sb, false, s, kk), idesc,
-                     (first && kk == 0) ? 0u : 1u);
+        const uint32_t s = 2u * (uint32_t)e, on = kt == k0 ? 0u : 1u;
+        const Desc a = desc_k(sa, s), b = desc_k(sb, s);
+        if (e == 64) mma_run<4>(acc, a, 0u, 2u, b, 0u, 2u, idesc, on);
+        else if (e == 32) mma_run<2>(acc, a, 0u, 2u, b, 0u, 2u, idesc, on);
+        else mma_run<1>(acc, a, 0u, 2u, b, 0u, 2u, idesc, on);
     }
 };
 
@@ -438,15 +480,14 @@ struct ConvStrip : ConvStore, TmaBase {
         u.ci = 0;
         return u;
     }
-    __device__ void issue(Cursor &u, const uint3 &, uint32_t sa, uint32_t sb, uint32_t bar) const {
+    __device__ void issue(Cursor &u, const uint3 &, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
         if (streamed) {
             // one strip (row y + dy, chunk ci) and the three taps' weight blocks
             const int c = u.ci * e;
-            if (c < c1) tma4(sa, &x1, c, u.x - 1, u.y + u.dy, u.b, bar);
-            else tma4(sa, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar);
+            if (lead) { if (c < c1) tma4(sa, &x1, c, u.x - 1, u.y + u.dy, u.b, bar); else tma4(sa, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar); }
             const uint32_t blk = (uint32_t)(bn * 2 * e);
             const int wk0 = (u.dy + 1) * 3 * C + c;  // tap (dy + 1) * 3 + (dx + 1)
-            for (int dx = 0; dx < 3; ++dx) tma2(sb + (uint32_t)dx * blk, &w, wk0 + dx * C, 0, bar);
+            for (int dx = 0; dx < 3; ++dx) if (lead) tma2(sb + (uint32_t)dx * blk, &w, wk0 + dx * C, 0, bar);
             if (++u.ci == nck) {
                 u.ci = 0;
                 ++u.dy;
@@ -455,30 +496,42 @@ struct ConvStrip : ConvStore, TmaBase {
         }
         uint32_t dst = sa;
         for (int ci = 0, c = 0; ci < nck; ++ci, c += e, dst += strip_bytes) {
-            if (c < c1) tma4(dst, &x1, c, u.x - 1, u.y + u.dy, u.b, bar);
-            else tma4(dst, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar);
+            if (lead) { if (c < c1) tma4(dst, &x1, c, u.x - 1, u.y + u.dy, u.b, bar); else tma4(dst, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar); }
         }
         ++u.dy;
     }
     __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt, int, const uint3 &,
                         uint32_t idesc) const {
-        const uint32_t S = 2u * (uint32_t)e, blk = (uint32_t)bn * S;
+        if (e == 64) mma_e<4>(acc, sa, sb, res, kt, idesc);
+        else if (e == 32) mma_e<2>(acc, sa, sb, res, kt, idesc);
+        else mma_e<1>(acc, sa, sb, res, kt, idesc);
+    }
+    // KK = e / 16 MMAs per tap and chunk; all offsets in descriptor units (16 bytes)
+    template <int KK>
+    __device__ __forceinline__ void mma_e(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt,
+                                          uint32_t idesc) const {
+        constexpr uint32_t S = 32u * KK, row = S / 16u;
+        const uint32_t blk = (uint32_t)bn * row;
+        uint32_t on = kt == 0 ? 0u : 1u;
+        const Desc a = desc_k(sa, S);
         if (streamed) {
+            const Desc b = desc_k(sb, S);
+#pragma unroll
             for (int dx = 0; dx < 3; ++dx)
-                for (int kk = 0; kk < e / 16; ++kk)
-                    mma_bf16(acc, op_desc(sa + (uint32_t)dx * S, false, S, kk),
-                             op_desc(sb + (uint32_t)dx * blk, false, S, kk), idesc,
-                             (kt == 0 && dx == 0 && kk == 0) ? 0u : 1u);
+                mma_run<KK>(acc, a, (uint32_t)dx * row, 2u, b, (uint32_t)dx * blk, 2u, idesc, dx ? 1u : on);
             return;
         }
-        uint32_t wb = res + (uint32_t)(kt * 3 * nck) * blk;  // tap kt*3 + dx
-        for (int dx = 0; dx < 3; ++dx)
-            for (int ci = 0; ci < nck; ++ci, wb += blk) {
-                const uint32_t a = sa + (uint32_t)ci * strip_bytes + (uint32_t)dx * S;
-                for (int kk = 0; kk < e / 16; ++kk)
-                    mma_bf16(acc, op_desc(a, false, S, kk), op_desc(wb, false, S, kk), idesc,
-                             (kt == 0 && dx == 0 && ci == 0 && kk == 0) ? 0u : 1u);
+        const Desc b = desc_k(res, S);
+        const uint32_t strip = strip_bytes >> 4;
+        uint32_t wb = (uint32_t)(kt * 3 * nck) * blk;  // tap kt*3 + dx
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+            uint32_t ao = (uint32_t)dx * row;
+            for (int ci = 0; ci < nck; ++ci, wb += blk, ao += strip) {
+                mma_run<KK>(acc, a, ao, 2u, b, wb, 2u, idesc, on);
+                on = 1u;
             }
+        }
     }
 };
 
@@ -520,15 +573,14 @@ struct WgradStrip : TmaBase {
         split_pixel(k0 * BK, H, W, u.b, u.y, u.x);
         return u;
     }
-    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar) const {
+    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
         uint32_t dst = sa;
         const int cg = (int)t.x * cpt * ea;  // first channel of this tile's chunk group
         for (int dyi = -1; dyi <= 1; ++dyi)
             for (int ci = 0, c = cg; ci < cpt; ++ci, c += ea, dst += strip_bytes) {
-                if (c < c1) tma4(dst, &x1, c, u.x - 1, u.y + dyi, u.b, bar);
-                else tma4(dst, &x2, c - c1, u.x - 1, u.y + dyi, u.b, bar);
+                if (lead) { if (c < c1) tma4(dst, &x1, c, u.x - 1, u.y + dyi, u.b, bar); else tma4(dst, &x2, c - c1, u.x - 1, u.y + dyi, u.b, bar); }
             }
-        for (int j = 0; j < nb; ++j) tma4(sb + (uint32_t)(j * 128 * eb), &dy, j * eb, u.x, u.y, u.b, bar);
+        for (int j = 0; j < nb; ++j) if (lead) tma4(sb + (uint32_t)(j * 128 * eb), &dy, j * eb, u.x, u.y, u.b, bar);
         u.x += BK;
         if (u.x == W) {
             u.x = 0;
@@ -540,22 +592,20 @@ struct WgradStrip : TmaBase {
     }
     __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt, int k0, const uint3 &t,
                         uint32_t idesc) const {
-        const bool first = kt == k0;
-        const uint32_t sA = 2u * (uint32_t)ea, sB = 2u * (uint32_t)eb;
-        uint32_t a0 = sa, accm = acc;
-        for (int st = 0; st < 3 * cpt; ++st, a0 += strip_bytes)
-            for (int h = 0; h < mtp; ++h, accm += (uint32_t)bn) {
-                const uint32_t start = a0 + (uint32_t)(2 * h) * sA;
-#pragma unroll
-                for (int kk = 0; kk < BK / 16; ++kk)
-                    mma_bf16(accm, sdesc_sw(start + (uint32_t)kk * 16u * sA, sA, 8u * sA, sA),
-                             op_desc(sb, true, sB, kk), idesc, (first && kk == 0) ? 0u : 1u);
+        const uint32_t sA = 2u * (uint32_t)ea, sB = 2u * (uint32_t)eb, on = kt == k0 ? 0u : 1u;
+        const Desc a = desc_sw(sa, sA, 8u * sA, sA), b = desc_mn(sb, sB);
+        const uint32_t strip = strip_bytes >> 4, half = sA >> 3;  // 2 sA bytes
+        uint32_t a0 = 0, accm = acc;
+        for (int st = 0; st < 3 * cpt; ++st, a0 += strip) {
+            mma_run<BK / 16>(accm, a, a0, sA, b, 0u, sB, idesc, on);
+            accm += (uint32_t)bn;
+            if (mtp == 2) {
+                mma_run<BK / 16>(accm, a, a0 + half, sA, b, 0u, sB, idesc, on);
+                accm += (uint32_t)bn;
             }
+        }
         if (t.x != 0) return;  // the bias row belongs to chunk group 0
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-            mma_bf16(accm, sdesc_sw(res + (uint32_t)kk * 16u * sA, sA, 8u * sA, sA), op_desc(sb, true, sB, kk),
-                     idesc, (first && kk == 0) ? 0u : 1u);
+        mma_run<BK / 16>(accm, desc_sw(res, sA, 8u * sA, sA), 0u, sA, b, 0u, sB, idesc, on);
     }
     __device__ void store(int row, int col, const float *v, const uint3 &t) const {
         const int m = col >> bn_shift, n = col & (bn - 1);
@@ -626,17 +676,16 @@ struct WgradTma : TmaBase {
         u.c0 = r0 - u.tap0 * C;
         return u;
     }
-    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar) const {
+    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
         const int R = 9 * C;
         int r = (int)t.x * BM, tap = u.tap0, c = u.c0;
         for (int j = 0; j < na; ++j, r += ea) {
             const uint32_t dst = sa + (uint32_t)(j * 128 * ea);
             if (r < R) {
                 const int dyy = tap / 3 - 1, dxx = tap % 3 - 1;
-                if (c < c1) tma4(dst, &x1, c, u.x + dxx, u.y + dyy, u.b, bar);
-                else tma4(dst, &x2, c - c1, u.x + dxx, u.y + dyy, u.b, bar);
+                if (lead) { if (c < c1) tma4(dst, &x1, c, u.x + dxx, u.y + dyy, u.b, bar); else tma4(dst, &x2, c - c1, u.x + dxx, u.y + dyy, u.b, bar); }
             } else if (r == R) {
-                tma2(dst, &ones, 0, 0, bar);
+                if (lead) tma2(dst, &ones, 0, 0, bar);
             }
             c += ea;
             if (c == C) {
@@ -645,7 +694,7 @@ struct WgradTma : TmaBase {
             }
         }
         for (int j = 0; j < nb; ++j)
-            tma4(sb + (uint32_t)(j * 128 * eb), &dy, (int)t.y * bn + j * eb, u.x, u.y, u.b, bar);
+            if (lead) tma4(sb + (uint32_t)(j * 128 * eb), &dy, (int)t.y * bn + j * eb, u.x, u.y, u.b, bar);
         // next 64 pixels: along the row (W >= 64), whole rows (py = 64 / W)
         // or whole images (pb = 64 / (H W))
         if (pb) {
@@ -670,12 +719,8 @@ struct WgradTma : TmaBase {
     __device__ void issue_res(uint32_t, uint32_t) const {}
     __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int k0, const uint3 &,
                         uint32_t idesc) const {
-        const bool first = kt == k0;
         const uint32_t s_a = 2u * (uint32_t)ea, s_b = 2u * (uint32_t)eb;
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-            mma_bf16(acc, op_desc(sa, true, s_a, kk), op_desc(sb, true, s_b, kk), idesc,
-                     (first && kk == 0) ? 0u : 1u);
+        mma_run<BK / 16>(acc, desc_mn(sa, s_a), 0u, s_a, desc_mn(sb, s_b), 0u, s_b, idesc, kt == k0 ? 0u : 1u);
     }
     __device__ void store(int row, int col, const float *v, const uint3 &t) const {
         const int R = 9 * C;
@@ -712,30 +757,27 @@ struct GemmTma : TmaBase {
     }
     struct Cursor { int k; };
     __device__ Cursor begin(const uint3 &, int k0) const { return Cursor{k0 * BK}; }
-    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar) const {
+    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
         if (!AMN) {
-            tma2(sa, &ma, u.k, (int)t.x * BM, bar);
+            if (lead) tma2(sa, &ma, u.k, (int)t.x * BM, bar);
         } else {
-            tma2(sa, &ma, (int)t.x * BM, u.k, bar);
-            tma2(sa + 8192u, &ma, (int)t.x * BM + 64, u.k, bar);
+            if (lead) tma2(sa, &ma, (int)t.x * BM, u.k, bar);
+            if (lead) tma2(sa + 8192u, &ma, (int)t.x * BM + 64, u.k, bar);
         }
         if (!BMN) {
-            tma2(sb, &mb, u.k, (int)t.y * bn, bar);
+            if (lead) tma2(sb, &mb, u.k, (int)t.y * bn, bar);
         } else {
             for (int j = 0; j < nb; ++j)
-                tma2(sb + (uint32_t)(j * 128 * eb), &mb, (int)t.y * bn + j * eb, u.k, bar);
+                if (lead) tma2(sb + (uint32_t)(j * 128 * eb), &mb, (int)t.y * bn + j * eb, u.k, bar);
         }
         u.k += BK;
     }
     __device__ void issue_res(uint32_t, uint32_t) const {}
     __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int k0, const uint3 &,
                         uint32_t idesc) const {
-        const bool first = kt == k0;
         const uint32_t s_b = BMN ? 2u * (uint32_t)eb : 128u;
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-            mma_bf16(acc, op_desc(sa, AMN, 128u, kk), op_desc(sb, BMN, s_b, kk), idesc,
-                     (first && kk == 0) ? 0u : 1u);
+        const Desc a = AMN ? desc_mn(sa, 128u) : desc_k(sa, 128u), b = BMN ? desc_mn(sb, s_b) : desc_k(sb, s_b);
+        mma_run<BK / 16>(acc, a, 0u, AMN ? 128u : 2u, b, 0u, BMN ? s_b : 2u, idesc, kt == k0 ? 0u : 1u);
     }
     __device__ void store(int row, int col, const float *v, const uint3 &t) const {
         const int m = (int)t.x * BM + row, n = (int)t.y * bn + col;
