@@ -26,7 +26,7 @@
 #include <vector>
 
 #include "kb_common.cuh"
-#include "kb_umma_tma.cuh"
+#include "kb_umma_roll.cuh"
 
 namespace kb {
 namespace sur {
@@ -436,13 +436,14 @@ struct Layer {
 // the one-CTA-per-tile engine.
 struct TmaPlan {
     int n = -1;
-    int f = 0, d = 0, w = 0;  // 0: per-tile engine, 1: TMA per-tap boxes, 2: TMA row strips
-    int wsplits = 0, wgroups = 1;
+    int f = 0, d = 0, w = 0;  // 0: per-tile engine, 1: TMA per-tap boxes, 2: row strips, 3: rolling rows
+    int wsplits = 0;
     int cp = 0;               // input channels of the weight-gradient partials (padded first layer: PAD_CH)
     kb::umma::ConvTma fwd, dgr;
     kb::umma::ConvStrip sfwd, sdgr;
+    kb::umma::ConvRoll rfwd, rdgr;
     kb::umma::WgradTma wg;
-    kb::umma::WgradStrip swg;
+    kb::umma::WgradRoll swg;
 };
 
 }  // namespace sur
@@ -528,19 +529,20 @@ void upsample(kb_surrogate *s, const Layer &l, int n, cudaStream_t st) {
                                                                               W, l.cin1);
 }
 
-// Row-strip weight gradient of a layer (input channels cin1 + cin2 in
-// chunks of ea): the chunks per tile (cpt, a divisor of the chunk count)
-// with the most MMA issuers per SM, the TMEM columns of a tile's
-// accumulators (all taps of its chunks plus the bias row) and the fit
-// (CTAs per SM); false when the layer does not take that form.
-struct StripWgradPlan { int ea, cpt, sr; uint32_t cols, strip, stage; kb::umma::TmaBase fit; };
-bool plan_strip_wgrad(const Layer &l, int W, int cin1, StripWgradPlan &P) {
+// Rolling row-strip weight gradient of a layer (input channels cin1 + cin2 in
+// chunks of ea): the chunks per CTA (cpt, a divisor of the chunk count) with
+// the most CTAs, so MMA issuers, per SM, the TMEM columns of a CTA's
+// accumulators (all taps of its chunks plus the bias row) and the CTAs per
+// SM; false when the layer does not take that form.  The ring holds the three
+// live rows and at least one more.
+struct RollWgradPlan { int ea, cpt, sr, cps; uint32_t cols, strip, stage, res; };
+bool plan_roll_wgrad(const Layer &l, int W, int cin1, RollWgradPlan &P) {
     using namespace kb::umma;
     const int ea = chunk_of(cin1, l.cin2), bn = l.bn_w;
     if (!ea || !chunk_of(bn) || W % BK || l.cout != bn || (bn & (bn - 1))) return false;
     const int nck = (cin1 + l.cin2) / ea, mtp = ea == 64 ? 2 : 1;
     const int sr = BK + (BM / ea - 1 > 3 ? BM / ea - 1 : 3);  // strip rows
-    const uint32_t strip = round1k((uint32_t)(sr * 2 * ea));
+    const uint32_t strip = round1k((uint32_t)(sr * 2 * ea)), res = (uint32_t)(72 * 2 * ea);
     bool found = false;
     for (int cpt = nck; cpt >= 1; --cpt) {
         if (nck % cpt) continue;
@@ -548,25 +550,25 @@ bool plan_strip_wgrad(const Layer &l, int W, int cin1, StripWgradPlan &P) {
         uint32_t cols = 32;
         while (cols < need) cols <<= 1;
         if (cols > 512) continue;
-        TmaBase b{};
-        b.a_bytes = 3u * (uint32_t)cpt * strip;
-        b.b_bytes = round1k((uint32_t)(bn * BK * 2));
-        b.res_bytes = (uint32_t)(72 * 2 * ea);
-        b.acc_cols = cols;
-        b.nbuf = 1;
-        // one CTA per SM (512 accumulator columns) measured slower than the
-        // per-tap boxes: take this form only where CTAs share the SM
-        if ((b.cps = tma_fit(b)) < 2) continue;
-        if (!found || b.cps > P.fit.cps) {
-            P = StripWgradPlan{ea, cpt, sr, cols, strip, b.a_bytes + b.b_bytes, b};
+        const uint32_t stage = (uint32_t)cpt * strip + round1k((uint32_t)(bn * BK * 2));
+        int cps = 0;
+        for (int k = TM_MAX_CPS; k >= 1 && !cps; --k)
+            if ((uint32_t)k * cols <= 512u && tma_stages(stage, res, k) >= 4) cps = k;
+        if (cps && (!found || cps > P.cps)) {
+            P = RollWgradPlan{ea, cpt, sr, cps, cols, strip, stage, res};
             found = true;
         }
     }
     return found;
 }
+// Pixel splits of that form: one CTA per (chunk group, split), all resident.
+int roll_wgrad_splits(const RollWgradPlan &P, int cin) {
+    const int groups = cin / P.ea / P.cpt, s = kb::sm_count() * P.cps / groups;
+    return s < 1 ? 1 : s;
+}
 
-// Row-strip convolution (forward or data gradient): input channels c1 + c2
-// in chunks of e, weights [Nout][Kp] resident, Nout one tile of bn.
+// Maps and shapes of a row-strip convolution (forward or data gradient): input
+// channels c1 + c2 in chunks of e, weights [Nout][Kp], Nout one tile of bn.
 int conv_strip(kb::umma::ConvStrip &c, const bf16 *x1, int c1, const bf16 *x2, int c2, const bf16 *wmat,
                int Kp, int bn, int e, int H, int W, int n, const char *what) {
     using namespace kb::umma;
@@ -589,42 +591,58 @@ int conv_strip(kb::umma::ConvStrip &c, const bf16 *x1, int c1, const bf16 *x2, i
     c.acc_cols = tmem_cols(bn);
     c.nbuf = 2;
     c.ncols = bn;
-    // resident weights, or streamed ones where that at least doubles the CTAs
-    // per SM (96-channel decoder input: 2 -> 4, 130 against 151 us; 3 -> 4
-    // measured slower: copying the weights per stage costs more)
-    c.streamed = 0;
-    c.tx = (uint32_t)(c.nck * (BM + 2) * 2 * e);
-    c.a_bytes = (uint32_t)c.nck * c.strip_bytes;
-    c.b_bytes = 0;
-    c.res_bytes = (uint32_t)(9 * c.nck * bn * 2 * e);
-    const int cps_res = tma_fit(c);
-    ConvStrip t = c;
-    t.streamed = 1;
-    t.tx = (uint32_t)((BM + 2) * 2 * e + 3 * bn * 2 * e);
-    t.a_bytes = c.strip_bytes;
-    t.b_bytes = round1k((uint32_t)(3 * bn * 2 * e));
-    t.res_bytes = 0;
-    const int cps_str = tma_fit(t);
-    if (cps_str >= 2 * cps_res) c = t;
-    c.cps = c.streamed ? cps_str : cps_res;
-    return c.cps ? 0 : kb::set_error(KB_ERR_ARG, "%s: row-strip convolution does not fit", what);
+    c.tx = (uint32_t)((BM + 2) * 2 * e + 3 * bn * 2 * e);
+    c.a_bytes = c.strip_bytes;
+    c.b_bytes = round1k((uint32_t)(3 * bn * 2 * e));
+    c.res_bytes = 0;
+    c.cps = tma_fit(c);
+    return 0;
 }
 
-// Whether a row-strip convolution of these shapes fits the engine.
+// The shared-memory and TMEM shape of the rolling form (roll_fit).
+void roll_shape(kb::umma::ConvRoll &r, int C, int e, int bn) {
+    using namespace kb::umma;
+    r.e = e;
+    r.C = C;
+    r.nck = C / e;
+    r.bn = r.ncols = bn;
+    r.strip_bytes = round1k((uint32_t)((BM + 2) * 2 * e));
+    r.tx = (uint32_t)((BM + 2) * 2 * e);
+    r.res_bytes = (uint32_t)(9 * r.nck * bn * 2 * e);
+    r.acc_cols = tmem_cols(bn);
+    r.cps = roll_fit(r);
+}
+
+// The rolling form of a row-strip convolution whose fields are set; false
+// where its weights leave no ring (streamed strips then).
+bool conv_roll(const kb::umma::ConvStrip &c, kb::umma::ConvRoll &r, int n) {
+    using namespace kb::umma;
+    r = ConvRoll{};
+    static_cast<ConvStore &>(r) = c;
+    r.x1 = c.x1;
+    r.x2 = c.x2;
+    r.w = c.w;
+    r.c1 = c.c1;
+    r.H = c.H;
+    r.W = c.W;
+    r.rows = n * (c.W / BM) * c.H;
+    roll_shape(r, c.C, c.e, c.bn);
+    return r.cps > 0;
+}
+
+// Whether a row-strip convolution of these shapes fits the engine, rolling or
+// with streamed weights.
 bool conv_strip_fits(int C, int e, int bn, int W) {
     using namespace kb::umma;
     if (!e || W % BM) return false;
-    TmaBase b{};
-    const int nck = C / e;
-    b.a_bytes = (uint32_t)nck * round1k((uint32_t)((BM + 2) * 2 * e));
-    b.res_bytes = (uint32_t)(9 * nck * bn * 2 * e);
-    b.acc_cols = tmem_cols(bn);
-    b.nbuf = 2;
-    TmaBase t = b;  // streamed weights
-    t.a_bytes = round1k((uint32_t)((BM + 2) * 2 * e));
+    ConvRoll r{};
+    roll_shape(r, C, e, bn);
+    TmaBase t{};
+    t.a_bytes = r.strip_bytes;
     t.b_bytes = round1k((uint32_t)(3 * bn * 2 * e));
-    t.res_bytes = 0;
-    return tma_fit(b) > 0 || tma_fit(t) > 0;
+    t.acc_cols = tmem_cols(bn);
+    t.nbuf = 2;
+    return r.cps > 0 || tma_fit(t) > 0;
 }
 
 // The network input (s->act[T_IN]) padded to PAD_CH channels (s->in_pad).
@@ -669,7 +687,7 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         c.relu = l.relu;
         c.out_f32 = l.out == T_OUT;
         c.store_cols = l.out == T_OUT ? 8 : 0;  // the head: the loss and unpacking read channels 0-2
-        p.f = 2;
+        p.f = conv_roll(c, p.rfwd, n) ? 3 : 2;
     } else if (ef && g128) {
         ConvTma &c = p.fwd;
         c = ConvTma{};
@@ -721,7 +739,7 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         c.bn = l.bn_d;
         c.relu = 0;
         c.out_f32 = 0;
-        p.d = 2;
+        p.d = conv_roll(c, p.rdgr, n) ? 3 : 2;
     } else if (i > 0 && ed && g128) {
         ConvTma &c = p.dgr;
         c = ConvTma{};
@@ -755,13 +773,13 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         c.out_f32 = 0;
         p.d = c.cps ? 1 : 0;
     }
-    // weight gradient: row strips (whole gradient per pixel split), or blocks
+    // weight gradient: rolling rows (whole gradient per pixel split), or blocks
     // of ea input channels / eb output-gradient channels x 64 pixels
     const int ea = chunk_of(cin1, l.cin2), eb = chunk_of(l.bn_w);
-    StripWgradPlan sp{};
-    if (eb && plan_strip_wgrad(l, W, cin1, sp)) {
-        WgradStrip &w = p.swg;
-        w = WgradStrip{};
+    RollWgradPlan sp{};
+    if (eb && plan_roll_wgrad(l, W, cin1, sp)) {
+        WgradRoll &w = p.swg;
+        w = WgradRoll{};
         const PixBox strip{sp.sr, 1, 1};
         if ((rc = nhwc_map(&w.x1, x1, cin1, W, H, n, ea, strip, what))) return rc;
         if (x2 && (rc = nhwc_map(&w.x2, x2, l.cin2, W, H, n, ea, strip, what))) return rc;
@@ -770,14 +788,10 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         const cuuint32_t bx[2] = {(cuuint32_t)ea, 72};
         if ((rc = bf16_map(&w.ones, s->ones, 2, d, sd, bx, 2 * ea, what))) return rc;
         if ((rc = nhwc_map(&w.dy, s->grad[l.out], l.cout, W, H, n, eb, b64, what))) return rc;
-        const int ngroups = cin / ea / sp.cpt;
-        const int nsteps = (M + BK - 1) / BK;
-        // about one tile (chunk group, pixel split) per CTA
-        int want = (kb::sm_count() * sp.fit.cps + ngroups - 1) / ngroups;
-        if (want > nsteps) want = nsteps;
-        const int sps = (nsteps + want - 1) / want;
-        p.wsplits = (nsteps + sps - 1) / sps;
-        p.wgroups = ngroups;
+        w.groups = cin / ea / sp.cpt;
+        w.nsteps = (M + BK - 1) / BK;
+        w.splits = std::min(roll_wgrad_splits(sp, cin), w.nsteps);
+        p.wsplits = w.splits;
         w.part = s->part + l.part_off;
         w.bn = l.bn_w;
         w.ea = ea;
@@ -787,8 +801,6 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         w.H = H;
         w.W = W;
         w.Nout = l.cout;
-        w.steps_per_split = sps;
-        w.nsteps = nsteps;
         w.cpt = sp.cpt;
         w.mtp = ea == 64 ? 2 : 1;
         w.nb = l.bn_w / eb;
@@ -796,15 +808,13 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         w.ea_shift = ea == 64 ? 6 : (ea == 32 ? 5 : 4);
         w.bn_shift = 31 - __builtin_clz((unsigned)l.bn_w);
         w.strip_bytes = sp.strip;
-        w.tx = (uint32_t)(3 * sp.cpt * sp.sr * 2 * ea + l.bn_w * BK * 2);
-        w.a_bytes = sp.fit.a_bytes;
-        w.b_bytes = sp.fit.b_bytes;
-        w.res_bytes = sp.fit.res_bytes;
+        w.tx = (uint32_t)(sp.sr * 2 * ea);  // one strip
+        w.stage_bytes = sp.stage;
+        w.res_bytes = sp.res;
         w.acc_cols = sp.cols;
-        w.nbuf = 1;  // about one tile per CTA: nothing to overlap the epilogue with
         w.ncols = (w.nmt + 1) * l.bn_w;
-        w.cps = tma_fit(w);
-        p.w = w.cps ? 2 : 0;
+        w.cps = sp.cps;
+        p.w = 3;
     } else if (ea && eb && g64) {
         WgradTma &w = p.wg;
         w = WgradTma{};
@@ -866,7 +876,8 @@ int forward(kb_surrogate *s, const void *input, int n, cudaStream_t st) {
             if (int rc = prepare_tma(s, i, n)) return rc;
             const TmaPlan &tp = s->tp[i];
             if (tp.f) {
-                if (int rc = tp.f == 2 ? launch_tma(tp.sfwd, grid, s->err, st)
+                if (int rc = tp.f == 3 ? launch_roll(tp.rfwd, s->err, st)
+                             : tp.f == 2 ? launch_tma(tp.sfwd, grid, s->err, st)
                                        : launch_tma(tp.fwd, grid, s->err, st))
                     return rc;
                 continue;
@@ -952,9 +963,9 @@ int backward(kb_surrogate *s, int n, cudaStream_t st) {
         // PAD_CH for the first layer)
         int sps = 0;
         int splits = wgrad_splits(l, M, sps);
-        if (tma && tp.w == 2) {
+        if (tma && tp.w == 3) {
             splits = tp.wsplits;
-            if (int rc = launch_tma(tp.swg, dim3(tp.wgroups, 1, splits), s->err, st)) return rc;
+            if (int rc = launch_wgrad_roll(tp.swg, s->err, st)) return rc;
         } else if (tma && tp.w == 1) {
             splits = tp.wsplits;
             const dim3 wg((9 * tp.cp + 1 + BM - 1) / BM, l.cout / l.bn_w, splits);
@@ -977,7 +988,8 @@ int backward(kb_surrogate *s, int n, cudaStream_t st) {
         // data gradient
         const dim3 grid((M + BM - 1) / BM, l.cin / l.bn_d);
         if (tma && tp.d) {
-            if (int rc = tp.d == 2 ? launch_tma(tp.sdgr, grid, s->err, st) : launch_tma(tp.dgr, grid, s->err, st))
+            if (int rc = tp.d == 3   ? launch_roll(tp.rdgr, s->err, st)
+                         : tp.d == 2 ? launch_tma(tp.sdgr, grid, s->err, st) : launch_tma(tp.dgr, grid, s->err, st))
                 return rc;
         } else {
             ConvOp op{};
@@ -1147,9 +1159,9 @@ int kb_surrogate_create(kb_surrogate **out, int max_batch, int H, int W, int bas
         const int cin1 = (l.in1 == T_IN && l.cin1 % 16) ? PAD_CH : l.cin1;
         const size_t E = (size_t)(9 * (cin1 + l.cin2) + 1) * l.cout;
         size_t need = (size_t)max_wgrad_splits(l) * E;
-        StripWgradPlan sp{};
-        if (plan_strip_wgrad(l, W >> l.level, cin1, sp))
-            need = std::max(need, (size_t)kb::sm_count() * kb::umma::TM_MAX_CPS * E);
+        RollWgradPlan rp{};
+        if (plan_roll_wgrad(l, W >> l.level, cin1, rp))
+            need = std::max(need, (size_t)roll_wgrad_splits(rp, cin1 + l.cin2) * E);
         // every layer's partials and grouped sums have their own region, so
         // the reductions of all layers run together after the backward pass
         l.part_off = part;

@@ -182,8 +182,8 @@ struct TmaBase {
 //   __device__ void prefetch()                     prefetch the tensor maps
 //   __device__ void issue_res(uint32_t res, uint32_t bar)   copies of the resident operand
 //   struct Cursor; __device__ Cursor begin(const uint3 &t, int k0)   state of step k0 of tile t
-//   __device__ void issue(Cursor &c, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar)
-//                                                  copies of the cursor's step; advance it
+//   __device__ void issue(Cursor &c, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead)
+//                                                  the lead lane's copies of the cursor's step; advance it
 //   __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt, int k0,
 //                       const uint3 &t, uint32_t idesc)   the MMAs of step kt of tile t
 template <class Op>
@@ -371,7 +371,7 @@ inline int tma_fit(const TmaBase &b) {
             return c;
     return 0;
 }
-constexpr size_t TM_SMEM_MAX = 1024 + TM_RING + (2 * TM_MAX_STAGES + 6) * 8 + 16;
+constexpr size_t TM_SMEM_MAX = 1024 + TM_RING + (2 * TM_MAX_STAGES + 10) * 8 + 16;
 
 // ---------------------------------------------------------------------------
 // Operations.
@@ -439,39 +439,29 @@ struct ConvTma : ConvStore, TmaBase {
 };
 
 // Convolution (forward or data gradient) of rows that are a multiple of 128
-// pixels wide, by row strips: a tile is 128 pixels of one row, a step is one
-// kernel row dy.  The step's copies are one strip per channel chunk, pixels
-// x0-1 .. x0+128 of row y+dy (box e x 130, K-major, swizzle 2e), so an
-// activation row crosses to shared memory three times instead of nine.  The
-// MMAs of tap dx read the strip from row dx+1 on: the tensor core applies the
-// swizzle to the absolute shared-memory address, so a start 2e bytes further
-// reads the rows shifted by one pixel.  The layer's weights (9 nck blocks of
-// bn x e, one output-channel tile) are the resident operand, in tap, chunk,
-// 16-wide K group order (the other engines' order); or, where that lets more
-// CTAs share an SM, they are streamed: a stage is then one kernel row and one
-// chunk, its strip and the three taps' weight blocks (order row, chunk, tap).
+// pixels wide, by row strips, for layers whose weights leave no room to stay
+// in shared memory (those that do roll down the rows, kb_umma_roll.cuh): a
+// tile is 128 pixels of one row, a step is one kernel row dy and one channel
+// chunk.  Its copies are one strip, pixels x0-1 .. x0+128 of row y+dy (box e x
+// 130, K-major, swizzle 2e), so an activation row crosses to shared memory
+// three times instead of nine, and the three taps' weight blocks (bn x e).
+// The MMAs of tap dx read the strip from row dx+1 on: the tensor core applies
+// the swizzle to the absolute shared-memory address, so a start 2e bytes
+// further reads the rows shifted by one pixel.
 struct ConvStrip : ConvStore, TmaBase {
     static constexpr bool A_MN = false, B_MN = false;
     CUtensorMap x1, x2, w;
     int e, c1, C, H, W, nck;
-    int streamed;  // 1: weights copied per stage (kernel row dy, chunk) instead of resident
     uint32_t strip_bytes, tx;
 
-    __device__ void k_range(const uint3 &, int &k0, int &k1) const {
-        k0 = 0;
-        k1 = streamed ? 3 * nck : 3;
-    }
+    __device__ void k_range(const uint3 &, int &k0, int &k1) const { k0 = 0; k1 = 3 * nck; }
     __device__ uint32_t step_tx(const uint3 &) const { return tx; }
     __device__ void prefetch() const {
         prefetch_map(&x1);
         if (c1 < C) prefetch_map(&x2);
         prefetch_map(&w);
     }
-    __device__ void issue_res(uint32_t res, uint32_t bar) const {
-        if (streamed) return;
-        const uint32_t blk = (uint32_t)(bn * 2 * e);
-        for (int j = 0, wk = 0; j < 9 * nck; ++j, wk += e) tma2(res + (uint32_t)j * blk, &w, wk, 0, bar);
-    }
+    __device__ void issue_res(uint32_t, uint32_t) const {}
     struct Cursor { int dy, ci, b, y, x; };
     __device__ Cursor begin(const uint3 &t, int) const {
         Cursor u;
@@ -481,155 +471,34 @@ struct ConvStrip : ConvStore, TmaBase {
         return u;
     }
     __device__ void issue(Cursor &u, const uint3 &, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
-        if (streamed) {
-            // one strip (row y + dy, chunk ci) and the three taps' weight blocks
+        if (lead) {
             const int c = u.ci * e;
-            if (lead) { if (c < c1) tma4(sa, &x1, c, u.x - 1, u.y + u.dy, u.b, bar); else tma4(sa, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar); }
+            if (c < c1) tma4(sa, &x1, c, u.x - 1, u.y + u.dy, u.b, bar);
+            else tma4(sa, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar);
             const uint32_t blk = (uint32_t)(bn * 2 * e);
             const int wk0 = (u.dy + 1) * 3 * C + c;  // tap (dy + 1) * 3 + (dx + 1)
-            for (int dx = 0; dx < 3; ++dx) if (lead) tma2(sb + (uint32_t)dx * blk, &w, wk0 + dx * C, 0, bar);
-            if (++u.ci == nck) {
-                u.ci = 0;
-                ++u.dy;
-            }
-            return;
+            for (int dx = 0; dx < 3; ++dx) tma2(sb + (uint32_t)dx * blk, &w, wk0 + dx * C, 0, bar);
         }
-        uint32_t dst = sa;
-        for (int ci = 0, c = 0; ci < nck; ++ci, c += e, dst += strip_bytes) {
-            if (lead) { if (c < c1) tma4(dst, &x1, c, u.x - 1, u.y + u.dy, u.b, bar); else tma4(dst, &x2, c - c1, u.x - 1, u.y + u.dy, u.b, bar); }
+        if (++u.ci == nck) {
+            u.ci = 0;
+            ++u.dy;
         }
-        ++u.dy;
     }
-    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt, int, const uint3 &,
+    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int, const uint3 &,
                         uint32_t idesc) const {
-        if (e == 64) mma_e<4>(acc, sa, sb, res, kt, idesc);
-        else if (e == 32) mma_e<2>(acc, sa, sb, res, kt, idesc);
-        else mma_e<1>(acc, sa, sb, res, kt, idesc);
+        if (e == 64) mma_e<4>(acc, sa, sb, kt, idesc);
+        else if (e == 32) mma_e<2>(acc, sa, sb, kt, idesc);
+        else mma_e<1>(acc, sa, sb, kt, idesc);
     }
-    // KK = e / 16 MMAs per tap and chunk; all offsets in descriptor units (16 bytes)
+    // KK = e / 16 MMAs per tap; all offsets in descriptor units (16 bytes)
     template <int KK>
-    __device__ __forceinline__ void mma_e(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt,
-                                          uint32_t idesc) const {
+    __device__ __forceinline__ void mma_e(uint32_t acc, uint32_t sa, uint32_t sb, int kt, uint32_t idesc) const {
         constexpr uint32_t S = 32u * KK, row = S / 16u;
-        const uint32_t blk = (uint32_t)bn * row;
-        uint32_t on = kt == 0 ? 0u : 1u;
-        const Desc a = desc_k(sa, S);
-        if (streamed) {
-            const Desc b = desc_k(sb, S);
+        const uint32_t blk = (uint32_t)bn * row, on = kt == 0 ? 0u : 1u;
+        const Desc a = desc_k(sa, S), b = desc_k(sb, S);
 #pragma unroll
-            for (int dx = 0; dx < 3; ++dx)
-                mma_run<KK>(acc, a, (uint32_t)dx * row, 2u, b, (uint32_t)dx * blk, 2u, idesc, dx ? 1u : on);
-            return;
-        }
-        const Desc b = desc_k(res, S);
-        const uint32_t strip = strip_bytes >> 4;
-        uint32_t wb = (uint32_t)(kt * 3 * nck) * blk;  // tap kt*3 + dx
-#pragma unroll
-        for (int dx = 0; dx < 3; ++dx) {
-            uint32_t ao = (uint32_t)dx * row;
-            for (int ci = 0; ci < nck; ++ci, wb += blk, ao += strip) {
-                mma_run<KK>(acc, a, ao, 2u, b, wb, 2u, idesc, on);
-                on = 1u;
-            }
-        }
-    }
-};
-
-// Weight gradient of rows that are a multiple of 64 pixels wide, one whole
-// gradient per tile: the tiles are the pixel splits, and a tile accumulates
-// every row r = tap C + c (and the bias row) in TMEM.  A step is 64 pixels
-// of one row.  Its copies are, per kernel row dy and channel chunk, one strip
-// of pixels x-1 .. x+sr-2 (box ea x sr, MN-major, swizzle 2ea), and the
-// step's output gradient (nb blocks of eb channels x 64 pixels), so each
-// input row crosses three times and each output-gradient row once.  M-tile m
-// = (dy, chunk, h) reads its strip with the blocks one row apart (LBO = 2ea
-// bytes): block j is the strip shifted by j pixels, i.e. tap dx = 2h - 1 + j
-// (blocks of taps beyond +1 are computed and not stored).  The bias M-tile
-// reads the resident `ones` rows (1 in channel 0).  Accumulator m holds
-// columns m bn .. m bn + bn - 1; the epilogue maps (m, row) to r.
-struct WgradStrip : TmaBase {
-    static constexpr bool A_MN = true, B_MN = true;
-    CUtensorMap x1, x2, ones, dy;
-    float *part;  // [splits][9C + 1][Nout]
-    int bn, ea, eb, c1, C, H, W, Nout, steps_per_split, nsteps;
-    int cpt, mtp, nb, nmt, ea_shift, bn_shift;  // chunks per tile, M-tiles per strip (1, 2), dY blocks, strip M-tiles
-    uint32_t strip_bytes, tx;
-
-    __device__ void k_range(const uint3 &t, int &k0, int &k1) const {
-        k0 = (int)t.z * steps_per_split;
-        k1 = min(nsteps, k0 + steps_per_split);
-    }
-    __device__ uint32_t step_tx(const uint3 &) const { return tx; }
-    __device__ void prefetch() const {
-        prefetch_map(&x1);
-        if (c1 < C) prefetch_map(&x2);
-        prefetch_map(&ones);
-        prefetch_map(&dy);
-    }
-    __device__ void issue_res(uint32_t res, uint32_t bar) const { tma2(res, &ones, 0, 0, bar); }
-    struct Cursor { int b, y, x; };
-    __device__ Cursor begin(const uint3 &, int k0) const {
-        Cursor u;
-        split_pixel(k0 * BK, H, W, u.b, u.y, u.x);
-        return u;
-    }
-    __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
-        uint32_t dst = sa;
-        const int cg = (int)t.x * cpt * ea;  // first channel of this tile's chunk group
-        for (int dyi = -1; dyi <= 1; ++dyi)
-            for (int ci = 0, c = cg; ci < cpt; ++ci, c += ea, dst += strip_bytes) {
-                if (lead) { if (c < c1) tma4(dst, &x1, c, u.x - 1, u.y + dyi, u.b, bar); else tma4(dst, &x2, c - c1, u.x - 1, u.y + dyi, u.b, bar); }
-            }
-        for (int j = 0; j < nb; ++j) if (lead) tma4(sb + (uint32_t)(j * 128 * eb), &dy, j * eb, u.x, u.y, u.b, bar);
-        u.x += BK;
-        if (u.x == W) {
-            u.x = 0;
-            if (++u.y == H) {
-                u.y = 0;
-                ++u.b;
-            }
-        }
-    }
-    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt, int k0, const uint3 &t,
-                        uint32_t idesc) const {
-        const uint32_t sA = 2u * (uint32_t)ea, sB = 2u * (uint32_t)eb, on = kt == k0 ? 0u : 1u;
-        const Desc a = desc_sw(sa, sA, 8u * sA, sA), b = desc_mn(sb, sB);
-        const uint32_t strip = strip_bytes >> 4, half = sA >> 3;  // 2 sA bytes
-        uint32_t a0 = 0, accm = acc;
-        for (int st = 0; st < 3 * cpt; ++st, a0 += strip) {
-            mma_run<BK / 16>(accm, a, a0, sA, b, 0u, sB, idesc, on);
-            accm += (uint32_t)bn;
-            if (mtp == 2) {
-                mma_run<BK / 16>(accm, a, a0 + half, sA, b, 0u, sB, idesc, on);
-                accm += (uint32_t)bn;
-            }
-        }
-        if (t.x != 0) return;  // the bias row belongs to chunk group 0
-        mma_run<BK / 16>(accm, desc_sw(res, sA, 8u * sA, sA), 0u, sA, b, 0u, sB, idesc, on);
-    }
-    __device__ void store(int row, int col, const float *v, const uint3 &t) const {
-        const int m = col >> bn_shift, n = col & (bn - 1);
-        const int R = 9 * C;
-        int r;
-        if (m == nmt) {
-            if (row != 0 || t.x != 0) return;
-            r = R;
-        } else {
-            const int st = mtp == 2 ? (m >> 1) : m, h = m - st * mtp;
-            const int dyi = st / cpt, ci = (int)t.x * cpt + st - dyi * cpt;
-            const int j = row >> ea_shift, c = row & (ea - 1);
-            const int dx = 2 * h - 1 + j;
-            if (dx > 1) return;
-            r = (dyi * 3 + dx + 1) * C + ci * ea + c;
-        }
-        float4 *d = reinterpret_cast<float4 *>(part + ((size_t)t.z * (R + 1) + r) * Nout + n);
-        d[0] = make_float4(v[0], v[1], v[2], v[3]);
-        d[1] = make_float4(v[4], v[5], v[6], v[7]);
-    }
-    struct Row { int r; };
-    __device__ Row row(int r, const uint3 &) const { return Row{r}; }
-    __device__ void store_row(const Row &R, int col, const float *v, const uint3 &t) const {
-        store(R.r, col, v, t);
+        for (int dx = 0; dx < 3; ++dx)
+            mma_run<KK>(acc, a, (uint32_t)dx * row, 2u, b, (uint32_t)dx * blk, 2u, idesc, dx ? 1u : on);
     }
 };
 
