@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(BX) fused_trt_libb_k(T *__restrict__ fo, const
 // The same step with the compact cut-link table: one class byte per node
 // replaces the solid mask and the 18 q_wall reads; link data are read only
 // at nodes with cut links.  Bit-identical to fused_trt_libb_k.  The update
-// of node c = (i, j, k) of class cl, shared by the node kernel and the
-// cut-node kernel so that both compute the same bits.
+// of node c = (i, j, k) of class cl, shared by the node blocks and the
+// cut-node blocks so that both compute the same bits.
 template <typename T, typename I>
 __device__ __forceinline__ void trt_links_node(T *__restrict__ fo, const T *__restrict__ fi,
                                                T *__restrict__ rho, T *__restrict__ ux,
@@ -294,18 +294,55 @@ __device__ __forceinline__ void trt_links_node(T *__restrict__ fo, const T *__re
     if (rho) { rho[c] = r; ux[c] = a_; uy[c] = b_; uz[c] = d_; }
 }
 
-// SKIP_CUT: class 2 nodes are left to fused_trt_cut_k, which runs beside
-// this kernel (the two write disjoint nodes and read only f_in), so this
-// kernel carries no link code.
-template <typename T, typename I, bool SKIP_CUT>
+// The cut node of record r of a compact table.
+template <typename T, typename I>
+__device__ __forceinline__ void trt_cut_node(T *__restrict__ fo, const T *__restrict__ fi,
+                                             T *__restrict__ rho, T *__restrict__ ux, T *__restrict__ uy,
+                                             T *__restrict__ uz, const LinkTable3 &L, const Grid3 &g, T sp,
+                                             T sm, long long r) {
+    if (r >= L.n_rec) return;
+    const size_t c = (size_t)L.node[r];
+    const size_t row = c / (size_t)g.Nx;
+    const int i = (int)(c - row * (size_t)g.Nx), j = (int)(row % (size_t)g.Ny),
+              k = (int)(row / (size_t)g.Ny);
+    trt_links_node<T, I>(fo, fi, rho, ux, uy, uz, L, g, sp, sm, c, i, j, k, 2);
+}
+// Record of a thread in the blocks of the first planes of the grid, which
+// take the cut nodes, one record per thread.
+__device__ __forceinline__ long long cut_record() {
+    return (((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * BX + threadIdx.x;
+}
+// Planes of the node grid that hold a table's records.
+inline unsigned cut_planes(const LinkTable3 &L, dim3 grid) {
+    const long long per = (long long)grid.x * grid.y * BX;
+    return (unsigned)((L.n_rec + per - 1) / per);
+}
+
+// zc > 0: the first zc planes of blocks update the table's cut nodes (class
+// 2), one record per thread, and the node blocks behind them skip those, so
+// they carry no divergent link code.  The two write disjoint nodes and read
+// only f_in.  As a kernel of their own the cut nodes needed a side stream with
+// a fork and a join event per step (192^3 FP32 step: 188.5 us, 183.0 with the
+// cut nodes in this grid).  zc = 0: link
+// code at every node.
+template <typename T, typename I, bool SPLIT>
 __global__ void __launch_bounds__(BX) fused_trt_links_k(T *__restrict__ fo, const T *__restrict__ fi,
                                                          T *__restrict__ rho, T *__restrict__ ux,
                                                          T *__restrict__ uy, T *__restrict__ uz,
-                                                         LinkTable3 L, Grid3 g, T sp, T sm) {
-    NODE3_IJK
+                                                         LinkTable3 L, Grid3 g, unsigned zc, T sp, T sm) {
+    int i, j;
+    const int k = (int)(blockIdx.z - (SPLIT ? zc : 0u));
+    if (SPLIT && k < 0) {
+        pdl_wait();
+        trt_cut_node<T, I>(fo, pdl_fresh(fi), rho, ux, uy, uz, L, g, sp, sm, cut_record());
+        return;
+    }
+    if (!node_ij(g.Nx, g.Ny, g.magic, i, j)) return;
+    pdl_wait();
+    fi = pdl_fresh(fi);
     const size_t c = (size_t)i + (size_t)g.Nx * ((size_t)j + (size_t)g.Ny * k);
-    const uint8_t cl = L.cls[c];
-    if (SKIP_CUT) {
+    const uint8_t cl = *pdl_fresh(L.cls + c);
+    if (SPLIT) {
         if (cl == 2) return;
         trt_links_node<T, I>(fo, fi, rho, ux, uy, uz, L, g, sp, sm, c, i, j, k, cl == 1 ? 1 : 0);
     } else {
@@ -316,8 +353,8 @@ __global__ void __launch_bounds__(BX) fused_trt_links_k(T *__restrict__ fo, cons
 // FP32 with even Nx and 8-byte aligned arrays: two adjacent nodes per thread,
 // each with the one-node kernel's scalar arithmetic, so the bits are the same.
 // CLS = false is fused_trt_k (cls: the solid mask or null), CLS = true is
-// fused_trt_links_k<SKIP_CUT> (cls: the table's class bytes; class 2 nodes are
-// left to fused_trt_cut_k).  Memory bound: the 8-byte accesses halve the
+// fused_trt_links_k<SPLIT> (cls: the table's class bytes; the first zc planes
+// of blocks take the cut nodes).  Memory bound: the 8-byte accesses halve the
 // stores and take a third off the loads (192^3 cut-link step 197.5 -> 188.5
 // us, 5.7 TB/s).
 template <bool CLS, typename I>
@@ -325,9 +362,15 @@ __global__ void __launch_bounds__(BX) fused_trt2_k(float *__restrict__ fo, const
                                                     float *__restrict__ rho, float *__restrict__ ux,
                                                     float *__restrict__ uy, float *__restrict__ uz,
                                                     const uint8_t *__restrict__ cls, Grid3 g,
-                                                    unsigned magic, float sp, float sm) {
+                                                    unsigned magic, float sp, float sm, LinkTable3 L,
+                                                    unsigned zc) {
     int i, j;
-    const int k = blockIdx.z;
+    const int k = (int)(blockIdx.z - (CLS ? zc : 0u));
+    if (CLS && k < 0) {
+        pdl_wait();
+        trt_cut_node<float, I>(fo, pdl_fresh(fi), rho, ux, uy, uz, L, g, sp, sm, cut_record());
+        return;
+    }
     if (!node_ij(g.Nx / 2, g.Ny, magic, i, j)) return;
     i *= 2;
     pdl_wait();
@@ -351,7 +394,7 @@ __global__ void __launch_bounds__(BX) fused_trt2_k(float *__restrict__ fo, const
     node(y, CLS ? cl.y == 1 : cl.y != 0, m[0].y, m[1].y, m[2].y, m[3].y);
     float *__restrict__ o0 = fo + c;
     if (CLS && (cl.x == 2 || cl.y == 2)) {
-        // one or both nodes belong to the cut-node kernel
+        // one or both nodes belong to the cut-node blocks
         if (cl.x != 2) {
 #pragma unroll
             for (int q = 0; q < 19; ++q) o0[q * P] = x[q];
@@ -382,31 +425,19 @@ inline bool pairs_fit(const Grid3 &g, const void *fo, const void *fi, const void
            al(cls, 2);
 }
 
+// L: the cut-link table (CLS), whose class bytes are cls; false where the grid
+// has no planes left for the cut nodes.
 template <bool CLS>
-void launch_trt2(float *fo, const float *fi, float *rho, float *ux, float *uy, float *uz,
-                 const uint8_t *cls, const Grid3 &g, float sp, float sm, cudaStream_t s) {
+bool launch_trt2(float *fo, const float *fi, float *rho, float *ux, float *uy, float *uz,
+                 const uint8_t *cls, const Grid3 &g, float sp, float sm, cudaStream_t s,
+                 const LinkTable3 &L = LinkTable3{}) {
     const auto k = offsets_fit_int(g, 19) ? fused_trt2_k<CLS, int> : fused_trt2_k<CLS, long long>;
-    const unsigned m = pair_magic(g);
-    // beside the cut-node kernel the launch follows an event wait: a plain one
-    if (CLS)
-        k<<<pair_grid(g), BX, 0, s>>>(fo, fi, rho, ux, uy, uz, cls, g, m, sp, sm);
-    else
-        launch_pdl(k, pair_grid(g), dim3(BX), s, fo, fi, rho, ux, uy, uz, cls, g, m, sp, sm);
-}
-
-// The cut nodes (class 2) of a compact table, one thread per record.
-template <typename T, typename I>
-__global__ void __launch_bounds__(BX) fused_trt_cut_k(T *__restrict__ fo, const T *__restrict__ fi,
-                                                       T *__restrict__ rho, T *__restrict__ ux,
-                                                       T *__restrict__ uy, T *__restrict__ uz,
-                                                       LinkTable3 L, Grid3 g, T sp, T sm) {
-    const long long r = (long long)blockIdx.x * BX + threadIdx.x;
-    if (r >= L.n_rec) return;
-    const size_t c = (size_t)L.node[r];
-    const size_t row = c / (size_t)g.Nx;
-    const int i = (int)(c - row * (size_t)g.Nx), j = (int)(row % (size_t)g.Ny),
-              k = (int)(row / (size_t)g.Ny);
-    trt_links_node<T, I>(fo, fi, rho, ux, uy, uz, L, g, sp, sm, c, i, j, k, 2);
+    dim3 grid = pair_grid(g);
+    const unsigned zc = CLS ? cut_planes(L, grid) : 0u;
+    if (grid.z + zc > 65535u) return false;
+    grid.z += zc;
+    launch_pdl(k, grid, dim3(BX), s, fo, fi, rho, ux, uy, uz, cls, g, pair_magic(g), sp, sm, L, zc);
+    return true;
 }
 
 // Cut-link table construction.  Pass 1 classifies every node and counts the
@@ -1567,29 +1598,19 @@ int build_links(kb_libb_links *L, const uint8_t *solid, const T *qw, const T *wx
 template <typename T, typename I>
 int launch_links_3d_i(T *fo, const T *fi, T *rho, T *ux, T *uy, T *uz,
                        const kb::d3::LinkTable3 &L, const Grid3 &g, T sp, T sm, cudaStream_t s) {
-    const dim3 grid = node_grid(g);
-    kb::d3::SideStream *ss = L.n_rec > 0 ? kb::d3::side_stream() : nullptr;
-    if (!ss) {  // no cut nodes, or no side stream: one kernel for every node
-        fused_trt_links_k<T, I, false><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
+    if constexpr (sizeof(T) == 4) {
+        if (pairs_fit(g, fo, fi, rho, ux, uy, uz, L.cls) &&
+            launch_trt2<true>(fo, fi, rho, ux, uy, uz, L.cls, g, sp, sm, s, L))
+            return KB_OK;
+    }
+    dim3 grid = node_grid(g);
+    const unsigned zc = kb::d3::cut_planes(L, grid);
+    if (grid.z + zc > 65535u) {  // no planes left for the cut nodes: link code at every node
+        kb::launch_pdl(fused_trt_links_k<T, I, false>, grid, dim3(BX), s, fo, fi, rho, ux, uy, uz, L, g, 0u, sp, sm);
         return KB_OK;
     }
-    // the cut nodes on the side stream, forked from s and joined back
-    // before anything that follows on s
-    cudaStream_t cs = s;
-    if (cudaEventRecord(ss->fork, s) == cudaSuccess && cudaStreamWaitEvent(ss->side, ss->fork, 0) == cudaSuccess)
-        cs = ss->side;
-    else
-        cudaGetLastError();
-    const unsigned nb = (unsigned)((L.n_rec + BX - 1) / BX);
-    fused_trt_cut_k<T, I><<<nb, BX, 0, cs>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
-    bool pairs = false;
-    if constexpr (sizeof(T) == 4) {
-        pairs = pairs_fit(g, fo, fi, rho, ux, uy, uz, L.cls);
-        if (pairs) launch_trt2<true>(fo, fi, rho, ux, uy, uz, L.cls, g, sp, sm, s);
-    }
-    if (!pairs) fused_trt_links_k<T, I, true><<<grid, BX, 0, s>>>(fo, fi, rho, ux, uy, uz, L, g, sp, sm);
-    if (cs != s && (cudaEventRecord(ss->join, cs) != cudaSuccess || cudaStreamWaitEvent(s, ss->join, 0) != cudaSuccess))
-        return kb::set_error(KB_ERR_CUDA, "kb_fused_trt_libb_links_step_3d: joining the cut-node stream failed");
+    grid.z += zc;
+    kb::launch_pdl(fused_trt_links_k<T, I, true>, grid, dim3(BX), s, fo, fi, rho, ux, uy, uz, L, g, zc, sp, sm);
     return KB_OK;
 }
 
