@@ -199,6 +199,21 @@ int kb_cavity_step_2d(void *f_out, const void *f_in, void *rho, void *ux, void *
                       const uint8_t *is_solid, int Nx, int Ny, double omega, double u_lid,
                       int dtype, void *stream);
 
+/* n_steps of kb_cavity_step_2d (moving_wall != 0: kb_cavity_movingwall_step_2d)
+ * in one launch, the populations in registers, with the bits of the step
+ * calls.  State 0 is read from f_0; the states n_steps - 1 and n_steps are left
+ * where alternating step calls leave them (state s in f_(s mod 2)); the moments
+ * are those of the last step.  `workspace` holds kb_cavity_run_bytes_2d bytes
+ * (16-byte aligned, contents ignored); its first int is 0 after a run and 1
+ * after one whose blocks gave up a wait for one another, whose results are
+ * void.  The launch is cooperative: kb_cavity_run_bytes_2d gives 0 bytes for a
+ * grid whose blocks are not all resident on the current device at once, and
+ * the run refuses it with KB_ERR_ARG.  KB_F64 or KB_F32. */
+int kb_cavity_run_bytes_2d(int Nx, int Ny, int moving_wall, int dtype, size_t *bytes);
+int kb_cavity_run_2d(void *f_0, void *f_1, void *rho, void *ux, void *uy, const uint8_t *is_solid,
+                     int Nx, int Ny, double omega, double u_lid, int moving_wall, int n_steps,
+                     void *workspace, size_t bytes, int dtype, void *stream);
+
 /* One consistent-initialisation iteration for the MRT cavity: the step of
  * kb_cavity_mrt_step_2d with the collision's velocity held at the given field
  * (ux, uy; double or float by fields_dtype) and the momentum reset to rho*u.

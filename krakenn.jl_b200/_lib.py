@@ -72,6 +72,8 @@ SIGNATURES: dict[str, list] = {
     "kb_cavity_mrt_init_step_2d": [_vp, _cvp, _cvp, _cvp, _i, _u8p, _i, _i, _d, _d, _d, _d, _d,
                                    _i, _vp],
     "kb_cavity_movingwall_step_2d": [_vp, _cvp, _vp, _vp, _vp, _u8p, _i, _i, _d, _d, _i, _vp],
+    "kb_cavity_run_bytes_2d": [_i, _i, _i, _i, C.POINTER(_sz)],
+    "kb_cavity_run_2d": [_vp, _vp, _vp, _vp, _vp, _u8p, _i, _i, _d, _d, _i, _i, _vp, _sz, _i, _vp],
     "kb_cavity_mrt_step_2d": [_vp, _cvp, _vp, _vp, _vp, _u8p, _i, _i, _d, _d, _d, _d, _d, _i,
                               _vp],
     "kb_fused_natconv_step": [_vp, _cvp, _vp, _cvp, _vp, _i, _i, _d, _d, _d, _d, _d, _d, _i, _vp],

@@ -684,6 +684,19 @@ __global__ void __launch_bounds__(BX) stream_px_wy_k(T *__restrict__ fo, const T
     for (int q = 0; q < 9; ++q) fo[c + q * P] = p[q];
 }
 
+// The stages after the pull of one run_cavity_2d step: zou_he_north (the lid
+// row only) -> collide_2d.
+template <typename T>
+__device__ __forceinline__ void cavity_node(T *p, bool lid, bool solid, T omega, T u_lid) {
+    if (lid) zou_he_north_node(p, u_lid);
+    if (solid) {
+        swap_pairs(p);
+    } else {
+        T r, a, b;
+        bgk(p, omega, r, a, b);
+    }
+}
+
 // One step of run_cavity_2d (src/drivers/basic.jl:121-136) in one launch.
 // stream_2d -> zou_he_north (row Ny only) -> collide_2d -> macroscopic on the
 // post-collision populations.  All stages after the pull touch only this node.
@@ -699,18 +712,33 @@ __global__ void __launch_bounds__(BX) cavity_step_k(T *__restrict__ fo, const T 
     solid = pdl_fresh(solid);
     T p[9];
     pull_bb(fi, g, i, j, p);
-    if (j == g.Ny - 1) zou_he_north_node(p, u_lid);
-    if (solid && solid[c]) {
-        swap_pairs(p);
-    } else {
-        T r, a, b;
-        bgk(p, omega, r, a, b);
-    }
+    cavity_node(p, j == g.Ny - 1, solid && solid[c], omega, u_lid);
 #pragma unroll
     for (int q = 0; q < 9; ++q) fo[c + q * P] = p[q];
     T r, a, b;
     macro_node(p, r, a, b);
     rho[c] = r; ux[c] = a; uy[c] = b;
+}
+
+// The stages after the pull of one step with the moving-wall lid; pull_bb has
+// already bounced the top row's links (p[4], p[7], p[8]).
+template <typename T>
+__device__ __forceinline__ void movingwall_node(T *p, bool lid, bool solid, T omega, T u_lid, T &r, T &a,
+                                                T &b) {
+    if (solid) {
+        swap_pairs(p);
+        r = T(1); a = T(0); b = T(0);
+    } else {
+        if (lid) {
+            const T d5 = -T(2.0 / 3.0) * T(0);
+            const T d8 = -T(1.0 / 6.0) * (u_lid + T(0));
+            const T d9 = -T(1.0 / 6.0) * (-u_lid + T(0));
+            p[4] = p[4] + d5;
+            p[7] = p[7] + d8;
+            p[8] = p[8] + d9;
+        }
+        bgk(p, omega, r, a, b);
+    }
 }
 
 // Lid-driven cavity step with a moving-wall half-way bounce-back lid: the
@@ -732,20 +760,7 @@ __global__ void __launch_bounds__(BX) cavity_movingwall_k(T *__restrict__ fo, co
     T p[9];
     pull_bb(fi, g, i, j, p);
     T r, a, b;
-    if (solid && solid[c]) {
-        swap_pairs(p);
-        r = T(1); a = T(0); b = T(0);
-    } else {
-        if (j == g.Ny - 1) {
-            const T d5 = -T(2.0 / 3.0) * T(0);
-            const T d8 = -T(1.0 / 6.0) * (u_lid + T(0));
-            const T d9 = -T(1.0 / 6.0) * (-u_lid + T(0));
-            p[4] = fi[c + 2 * P] + d5;
-            p[7] = fi[c + 5 * P] + d8;
-            p[8] = fi[c + 6 * P] + d9;
-        }
-        bgk(p, omega, r, a, b);
-    }
+    movingwall_node(p, j == g.Ny - 1, solid && solid[c], omega, u_lid, r, a, b);
 #pragma unroll
     for (int q = 0; q < 9; ++q) fo[c + q * P] = p[q];
     if (rho) { rho[c] = r; ux[c] = a; uy[c] = b; }
@@ -1265,6 +1280,8 @@ __global__ void __launch_bounds__(BX) forced2_k(float *__restrict__ f, const flo
 }  // namespace d2
 }  // namespace kb
 
+#include "kb_resident2d.cuh"
+
 // ----------------------------------------------------------- host wrappers --
 namespace {
 
@@ -1623,6 +1640,36 @@ int kb_cavity_step_2d(void *f_out, const void *f_in, void *rho, void *ux, void *
         (kb::launch_pdl(cavity_step_k<T>, nodes_grid(Nx, Ny), dim3(BX), kb::as_stream(stream),
             (T *)f_out, (const T *)f_in, (T *)rho, (T *)ux, (T *)uy, is_solid, grid2<T>(Nx, Ny),
             (T)omega, (T)u_lid)));
+}
+
+int kb_cavity_run_bytes_2d(int Nx, int Ny, int moving_wall, int dtype, size_t *bytes) {
+    KB_REQUIRE(bytes, "kb_cavity_run_bytes_2d: null pointer");
+    *bytes = 0;
+    if (int e = check_dims("kb_cavity_run_bytes_2d", Nx, Ny)) return e;
+    KB_DISPATCH_PLAIN("kb_cavity_run_bytes_2d", dtype,
+        *bytes = moving_wall ? (cavity_run_bytes<T, true>(Nx, Ny)) : (cavity_run_bytes<T, false>(Nx, Ny)));
+}
+
+int kb_cavity_run_2d(void *f_0, void *f_1, void *rho, void *ux, void *uy, const uint8_t *is_solid,
+                     int Nx, int Ny, double omega, double u_lid, int moving_wall, int n_steps,
+                     void *workspace, size_t bytes, int dtype, void *stream) {
+    const char *what = "kb_cavity_run_2d";
+    KB_REQUIRE(f_0 && f_1 && rho && ux && uy && workspace, "%s: null pointer", what);
+    KB_REQUIRE(f_0 != f_1, "%s: f_0 and f_1 must differ", what);
+    KB_REQUIRE(n_steps >= 1, "%s: n_steps must be positive (got %d)", what, n_steps);
+    KB_REQUIRE((uintptr_t)workspace % 16 == 0, "%s: the workspace must be 16-byte aligned", what);
+    if (int e = check_dims(what, Nx, Ny)) return e;
+    KB_DISPATCH_PLAIN(what, dtype,
+        CavityRun<T> R = {};
+        R.f0 = (T *)f_0; R.f1 = (T *)f_1;
+        R.rho = (T *)rho; R.ux = (T *)ux; R.uy = (T *)uy;
+        R.solid = is_solid;
+        R.Nx = Nx; R.Ny = Ny; R.nsteps = (unsigned)n_steps;
+        R.omega = (T)omega; R.u_lid = (T)u_lid;
+        cudaStream_t s = kb::as_stream(stream);
+        const int rc = moving_wall ? (cavity_run<T, true>(what, R, workspace, bytes, s))
+                                   : (cavity_run<T, false>(what, R, workspace, bytes, s));
+        if (rc) return rc);
 }
 
 int kb_cavity_mrt_step_2d(void *f_out, const void *f_in, void *rho, void *ux, void *uy,

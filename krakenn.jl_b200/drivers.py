@@ -114,6 +114,8 @@ def run_cavity_2d(config: LBMConfig, backend="b200", T=torch.float64, fused=True
     kb_cavity_step_2d, which gives the same bits.
     lid="moving_wall": half-way bounce-back on all four walls with the
     moving-wall link rule on the lid (kb_cavity_movingwall_step_2d).
+    Without on_step, a grid that is resident on the device at once (about
+    256^2) runs all its steps in one launch (kb_cavity_run_2d, same bits).
     on_step(step, fields): called after every step with the device moment
     fields (for example an output.StepOutput)."""
     _require_backend(backend)
@@ -140,12 +142,25 @@ def run_cavity_2d(config: LBMConfig, backend="b200", T=torch.float64, fused=True
             ops.collide_2d_(fo, solid, w)
             ops.compute_macroscopic_2d_(rho, ux, uy, fo)
 
+    ws = None
     if on_step is None:
-        _step_loop(step, config.max_steps, True)
+        moving = lid == "moving_wall"
+        # short runs, and grids whose blocks are not all resident at once, take the step loop
+        nb = 0
+        if (fused or moving) and config.max_steps >= 2 * _CYCLE:
+            nb = ops.cavity_run_bytes_2d(Nx, Ny, moving, f_in.dtype)
+        if nb:
+            ws = torch.empty((nb + 3) // 4, dtype=torch.int32, device=f_in.device)
+            ops.cavity_run_2d_(f[0], f[1], rho, ux, uy, solid, Nx, Ny, w, config.u_lid, moving,
+                               config.max_steps, ws)
+        else:
+            _step_loop(step, config.max_steps, True)
     else:
         for n in range(config.max_steps):
             step(n & 1)
             on_step(n + 1, {"rho": rho, "velocity": (ux, uy)})
+    if ws is not None and int(ws[0]):
+        raise RuntimeError("run_cavity_2d: the run gave up a wait between its blocks")
     st["f_in"], st["f_out"] = f[config.max_steps & 1], f[1 - (config.max_steps & 1)]
     return dict(rho=rho.cpu().numpy(), ux=ux.cpu().numpy(), uy=uy.cpu().numpy(), config=config,
                 state=st)

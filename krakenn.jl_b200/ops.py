@@ -384,6 +384,33 @@ def cavity_mrt_step_2d_(f_out, f_in, rho, ux, uy, is_solid, Nx, Ny, nu, u_lid, s
          float(s_eps), float(s_q), float(u_lid), code, _stream())
 
 
+def cavity_run_bytes_2d(Nx, Ny, moving_wall, dtype):
+    """Workspace bytes of cavity_run_2d_; 0 if the grid is too large to be
+    resident on the device at once."""
+    n = C.c_size_t(0)
+    call("kb_cavity_run_bytes_2d", Nx, Ny, int(bool(moving_wall)),
+         KB_F64 if dtype == torch.float64 else KB_F32, C.byref(n))
+    return n.value
+
+
+def cavity_run_2d_(f_0, f_1, rho, ux, uy, is_solid, Nx, Ny, omega, u_lid, moving_wall, n_steps,
+                   workspace):
+    """n_steps of cavity_step_2d_ (moving_wall: cavity_movingwall_step_2d_) in
+    one launch; state s is left in f_(s mod 2) for the last two steps.
+    workspace: int32 tensor of cavity_run_bytes_2d bytes; its first value is
+    not 0 after a run that failed."""
+    code = _plain(f_0)
+    if f_1.dtype != f_0.dtype:
+        raise _arg_error(f"f_1 must be a {f_0.dtype} tensor")
+    if workspace.dtype != torch.int32:
+        raise _arg_error("workspace must be an int32 tensor")
+    _match2(f_0, Nx, Ny); _match2(f_1, Nx, Ny)
+    _ptrs_2d_fields(code, Nx, Ny, rho=rho, ux=ux, uy=uy)
+    call("kb_cavity_run_2d", _t(f_0, "f_0"), _t(f_1, "f_1"), _t(rho, "rho"), _t(ux, "ux"),
+         _t(uy, "uy"), _mask(is_solid), Nx, Ny, float(omega), float(u_lid), int(bool(moving_wall)),
+         int(n_steps), _t(workspace, "workspace"), workspace.numel() * 4, code, _stream())
+
+
 def rayleigh_step_2d_(f_out, f_in, g_out, g_in, Nx, Ny, omega_f, omega_T, beta_g, T_ref, T_hot,
                       T_cold, vertical):
     """One run_rayleigh_benard_2d step (src/drivers/thermal.jl:101-130) in one
