@@ -609,7 +609,8 @@ void roll_shape(kb::umma::ConvRoll &r, int C, int e, int bn) {
     r.strip_bytes = round1k((uint32_t)((BM + 2) * 2 * e));
     r.tx = (uint32_t)((BM + 2) * 2 * e);
     r.res_bytes = (uint32_t)(9 * r.nck * bn * 2 * e);
-    r.acc_cols = tmem_cols(bn);
+    r.tmem_cols = 32;
+    while (r.tmem_cols < (uint32_t)(ROLL_ACC * bn)) r.tmem_cols *= 2;
     r.cps = roll_fit(r);
 }
 

@@ -18,6 +18,14 @@ namespace umma {
 // a single tile, and bytes in flight over latency bound the layer (32 channels,
 // 256^2, batch 16: 50 us against 20 us of HBM traffic).  The batch-16 256^2
 // network: inference 734 -> 674 us, gradient 2482 -> 2383 us.
+// The three kernel rows of a tap share one MMA: their weight blocks lie one
+// after another in shared memory (kernel rows 2, 1, 0) and their output rows in
+// neighbouring accumulators, bn columns apart, so an N of 3 bn reads the strip
+// once where three MMAs read it three times (an MMA of N = 32 is bound by
+// reading its 4 KB A operand).  The ring splits a run where it wraps, the row
+// that starts from 0 is a run of its own on the first tap, and N stops at 256.
+// The 96-channel decoder layer's forward 95 -> 73 us, the 32-channel layers 2 to
+// 5 us less; inference 671 -> 642 us, gradient 2335 -> 2310 us.
 // The epilogue loads the row's ReLU mask while the accumulator is still being
 // computed and reads 16 TMEM columns per wait.
 struct ConvRoll : ConvStore {
@@ -25,7 +33,7 @@ struct ConvRoll : ConvStore {
     int e, c1, C, H, W, nck;
     int rows;                          // row tiles: images x W / 128 x H
     uint32_t strip_bytes, tx;          // a ring stage: one chunk of one input row
-    uint32_t res_bytes, acc_cols;      // resident weights; TMEM columns of one accumulator
+    uint32_t res_bytes, tmem_cols;     // resident weights; TMEM columns of the accumulators, bn apart
     int ncols, cps;
 };
 constexpr int ROLL_ACC = 4;
@@ -79,11 +87,11 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
     uint64_t *resbar = drain + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(resbar + 1);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    const uint32_t cols = op.acc_cols;
+    const uint32_t cols = (uint32_t)op.bn;
 
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)ROLL_ACC * cols));
+                     ::"r"(smem_u32(tmem_slot)), "r"(op.tmem_cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
@@ -114,8 +122,11 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
             prefetch_map(&op.w);
             const uint32_t blk = (uint32_t)(op.bn * 32 * KK);
             expect_tx(smem_u32(resbar), op.res_bytes);
-            for (int j = 0; j < 9 * op.nck; ++j)
-                tma2(res + (uint32_t)j * blk, &op.w, j * 16 * KK, 0, smem_u32(resbar));
+            // (dx, chunk) blocks of the kernel rows 2, 1, 0, one after another
+            for (int j = 0; j < 9 * op.nck; ++j) {
+                const int k = j % 3, g = j / 3, dx = g / op.nck, ci = g - dx * op.nck;
+                tma2(res + (uint32_t)j * blk, &op.w, (((2 - k) * 3 + dx) * op.nck + ci) * 16 * KK, 0, smem_u32(resbar));
+            }
         }
         long long g = 0;
         int s = 0;
@@ -149,7 +160,8 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
         if (!mbar_wait_warp(resbar, 0u, spin)) ok = false;
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
-        const uint32_t idesc = idesc_bf16(op.bn, false, false);
+        const uint32_t idesc1 = idesc_bf16(op.bn, false, false), idesc_step = idesc_bf16(2 * op.bn, false, false) - idesc1;
+        const int gmax = 256 / op.bn;
         constexpr uint32_t S = 32u * KK, row = S / 16u;
         const uint32_t blk = (uint32_t)op.bn * row;
         const Desc bw = desc_k(res, S);
@@ -170,19 +182,20 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elect_one()) {
                         const Desc a = desc_k(base + (uint32_t)s * stage_bytes, S);
+                        // kernel row 2 - o feeds output row t - 1 + o; rows in
+                        // neighbouring accumulators share one MMA
+                        const int o0 = max(0, seg.ya - t + 1), o1 = min(2, seg.yb - t);
 #pragma unroll
-                        for (int kr = 2; kr >= 0; --kr) {  // output row y = t + 1 - kr
-                            const int y = t + 1 - kr;
-                            if (y < seg.ya || y >= seg.yb) continue;
-                            const uint32_t acc = tmem + (uint32_t)((n + 1 - kr) % ROLL_ACC) * cols;
-                            uint32_t on = kr == 0 && ci == 0 ? 0u : 1u;
-#pragma unroll
-                            for (int dx = 0; dx < 3; ++dx) {
-                                mma_run<KK>(acc, a, (uint32_t)dx * row, 2u, bw,
-                                            (uint32_t)((kr * 3 + dx) * op.nck + ci) * blk, 2u, idesc, on);
-                                on = 1u;
+                        for (int dx = 0; dx < 3; ++dx)
+                            for (int o = o0; o <= o1;) {
+                                const int slot = (n - 1 + o) % ROLL_ACC;
+                                const bool first = dx == 0 && ci == 0;  // row t + 1 starts from 0
+                                const int run = min(min((first && o < 2 ? min(o1, 1) : o1) + 1 - o, ROLL_ACC - slot), gmax);
+                                mma_run<KK>(tmem + (uint32_t)slot * cols, a, (uint32_t)dx * row, 2u, bw,
+                                            (uint32_t)((dx * op.nck + ci) * 3 + o) * blk, 2u, idesc1 + (uint32_t)(run - 1) * idesc_step,
+                                            first && o == 2 ? 0u : 1u);
+                                o += run;
                             }
-                        }
                         mma_commit(&empty[s]);
                         if (ci == op.nck - 1 && t - 1 >= seg.ya) mma_commit(&acc_full[(n - 1) % ROLL_ACC]);
                     }
@@ -276,7 +289,7 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
     __syncthreads();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"((uint32_t)ROLL_ACC * cols));
+                     "r"(op.tmem_cols));
 }
 
 // Weight gradient of rows that are a multiple of 64 pixels wide, rolling down
@@ -521,7 +534,7 @@ inline size_t roll_smem_bytes(const ConvRoll &c, int ns) {
 inline int roll_fit(const ConvRoll &c) {
     const int nq = (c.ncols + 31) / 32, most = nq == 1 ? 4 : (nq == 2 ? 2 : 1);
     for (int k = most; k >= 1; --k)
-        if ((uint32_t)(k * ROLL_ACC) * c.acc_cols <= 512u && roll_stages(c, k) >= 2) return k;
+        if ((uint32_t)k * c.tmem_cols <= 512u && roll_stages(c, k) >= 2) return k;
     return 0;
 }
 
@@ -545,7 +558,7 @@ int launch_roll_t(const ConvRoll &c, int *err, cudaStream_t stream, long long sp
 inline int launch_roll(const ConvRoll &c, int *err, cudaStream_t stream, long long spin = 1ll << 22) {
     const int nq = (c.ncols + 31) / 32;
     if (c.cps < 1 || c.cps > TM_MAX_CPS || roll_stages(c, c.cps) < 2 || nq > 4 || c.rows < 1 ||
-        (uint32_t)(c.cps * ROLL_ACC) * c.acc_cols > 512u || c.ncols > (int)c.acc_cols)
+        (uint32_t)c.cps * c.tmem_cols > 512u || (uint32_t)(ROLL_ACC * c.bn) > c.tmem_cols)
         return kb::set_error(KB_ERR_ARG, "conv_roll_k: shape does not fit");
 #define KB_ROLL(KK)                                                                          \
     do {                                                                                     \
