@@ -270,7 +270,7 @@ struct RJob {
     const float *part;
     float *tmp, *gW, *gb;
     int splits, groups, per, E, Cp, Cs, cout;
-    long long g_start, r_start;  // first work item of the job in each pass
+    long long g_start, r_start;  // first work item (four elements) of the job in each pass
 };
 constexpr int N_LAYERS_MAX = 16;  // >= N_LAYERS
 static_assert(N_LAYERS <= N_LAYERS_MAX, "job tables hold every layer");
@@ -280,38 +280,62 @@ struct RJobs {
     long long g_total, r_total;
 };
 
+// Four elements per thread (cout is a multiple of 16, so E of 4) and four
+// splits in flight: the partials, about 290 MB at batch 16, are read once and
+// bound both passes.  With one element per thread and scattered single writes
+// the passes took 69 and 30 us, with these 42 and 23; gradient 2301 -> 2260 us.
+__device__ __forceinline__ float4 sum_splits(const float *src, size_t E, int n) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int z = 0; z < n; ++z) {
+        const float4 v = __ldcs(reinterpret_cast<const float4 *>(src + (size_t)z * E));
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    return s;
+}
+
 __global__ void wgrad_group_all_k(const RJobs J) {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < J.g_total;
          t += (long long)gridDim.x * blockDim.x) {
         int k = 0;
         while (k + 1 < J.n && t >= J.j[k + 1].g_start) ++k;
         const RJob &b = J.j[k];
-        const int u = (int)(t - b.g_start), g = u / b.E, e = u - g * b.E;
+        const int u = (int)(t - b.g_start), E4 = b.E >> 2, g = u / E4, e = (u - g * E4) * 4;
         const int z0 = g * b.per, z1 = min(b.splits, z0 + b.per);
-        float s = 0.f;
-        for (int z = z0; z < z1; ++z) s += b.part[(size_t)z * b.E + e];
-        b.tmp[(size_t)g * b.E + e] = s;
+        *reinterpret_cast<float4 *>(b.tmp + (size_t)g * b.E + e) =
+            sum_splits(b.part + (size_t)z0 * b.E + e, b.E, z1 - z0);
     }
 }
 
+// A warp takes 8 input channels x 16 output channels of a tap, so that its
+// reads (64 bytes of a row) and its transposed writes (8 channels of gW[cout])
+// are whole sectors; the bias row has quads of its own behind them.
 __global__ void wgrad_reduce_all_k(const RJobs J) {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < J.r_total;
          t += (long long)gridDim.x * blockDim.x) {
         int k = 0;
         while (k + 1 < J.n && t >= J.j[k + 1].r_start) ++k;
         const RJob &b = J.j[k];
-        const int e = (int)(t - b.r_start);
+        const int u = (int)(t - b.r_start), nw = (9 * b.Cp * b.cout) >> 2;
         const float *src = b.groups > 1 ? b.tmp : b.part;
         const int nz = b.groups > 1 ? b.groups : b.splits;
-        float s = 0.f;
-        for (int z = 0; z < nz; ++z) s += src[(size_t)z * b.E + e];
-        const int Rp = 9 * b.Cp, r = e / b.cout, co = e - r * b.cout;
-        if (r == Rp) {
-            b.gb[co] = s;
-        } else {
-            const int tap = r / b.Cp, c = r - tap * b.Cp;
-            if (c < b.Cs) b.gW[((size_t)co * 9 + tap) * b.Cs + c] = s;
+        if (u >= nw) {
+            if (u >= b.E >> 2) continue;
+            const float4 s = sum_splits(src + (size_t)nw * 4 + (size_t)(u - nw) * 4, b.E, nz);
+            *reinterpret_cast<float4 *>(b.gb + (u - nw) * 4) = s;
+            continue;
         }
+        const int blk = u >> 5, ncb = b.cout >> 4, rb = blk / ncb;  // 16 output channels fastest
+        const int co = (blk - rb * ncb) * 16 + (u & 3) * 4, r = rb * 8 + ((u >> 2) & 7);
+        const float4 s = sum_splits(src + (size_t)r * b.cout + co, b.E, nz);
+        const int tap = r / b.Cp, c = r - tap * b.Cp;
+        if (c >= b.Cs) continue;
+        float *o = b.gW + ((size_t)co * 9 + tap) * b.Cs + c;
+        const size_t step = (size_t)9 * b.Cs;
+        o[0] = s.x;
+        o[step] = s.y;
+        o[2 * step] = s.z;
+        o[3 * step] = s.w;
     }
 }
 
@@ -929,8 +953,8 @@ void add_reduce_job(kb_surrogate *s, RJobs &J, const Layer &l, int splits, int C
     b.cout = l.cout;
     b.g_start = J.g_total;
     b.r_start = J.r_total;
-    if (groups > 1) J.g_total += groups * E;
-    J.r_total += E;
+    if (groups > 1) J.g_total += groups * E / 4;
+    J.r_total += (E / 4 + 31) / 32 * 32;  // whole warps per job
 }
 
 void run_reduce_jobs(const RJobs &J, cudaStream_t st) {
