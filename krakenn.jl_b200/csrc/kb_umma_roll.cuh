@@ -26,8 +26,13 @@ namespace umma {
 // that starts from 0 is a run of its own on the first tap, and N stops at 256.
 // The 96-channel decoder layer's forward 95 -> 73 us, the 32-channel layers 2 to
 // 5 us less; inference 671 -> 642 us, gradient 2335 -> 2310 us.
-// The epilogue loads the row's ReLU mask while the accumulator is still being
-// computed and reads 16 TMEM columns per wait.
+// The epilogue reads 16 TMEM columns per wait.  A lane is a pixel, so an access
+// of a warp touches up to 32 lines whatever its width, and the load-store unit
+// bounds the epilogue: masks and outputs move 32 bytes per access (the 96-channel
+// data gradient 120 -> 92 us, 32 -> 32 channels forward 36 -> 31; inference 640 ->
+// 607 us, gradient 2255 -> 2171).  The ReLU mask of a row is loaded while the
+// accumulator is still being computed, with more than 32 columns one row ahead
+// (2171 -> 2155 us; with four CTAs per SM there are no registers for it).
 struct ConvRoll : ConvStore {
     CUtensorMap x1, x2, w;
     int e, c1, C, H, W, nck;
@@ -49,6 +54,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 32 bytes of one pixel (16 channels) in one access.
+__device__ __forceinline__ void ld32(uint32_t *r, const void *p) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void st32(void *p, const uint32_t *r) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 
 // A CTA's range of row tiles as segments of one column: rows [ya, yb) of the
@@ -216,22 +233,34 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
         const int q = warp & 3, grp = (warp - 2) >> 2;
         const int px = q * 32 + lane;
         int n = 0;
+        // the ReLU mask of the warp's columns at pixel x of row y
+        auto load_mask = [&](int x, int y, uint32_t (*mk)[8]) {
+            const int up = op.mask.up1;
+            const size_t m = ((size_t)seg.b * op.H + y) * op.W + x;
+            const __nv_bfloat16 *m1 =
+                op.mask.s1 + (((size_t)seg.b * (op.H >> up) + (y >> up)) * (op.W >> up) + (x >> up)) * op.mask.c1;
+            const __nv_bfloat16 *m2 = op.mask.s2 ? op.mask.s2 + m * op.mask.c2 - op.mask.c1 : m1;
+#pragma unroll
+            for (int g = 0; g < NQ; ++g) {
+                const int c16 = g * 16 * TM_EPI + grp * 16;
+                if (c16 < op.ncols) ld32(mk[g], (c16 < op.mask.c1 ? m1 : m2) + c16);
+            }
+        };
+        uint32_t mk[NQ][8], next[NQ][8];
         while (ok && seg.next(op))
             for (int y = seg.ya; y < seg.yb; ++y, ++n) {
                 const int x = seg.x0 + px;
                 const size_t m = ((size_t)seg.b * op.H + y) * op.W + x;
-                uint4 mk[2 * NQ];
                 if (op.mask.s1) {
-                    const int up = op.mask.up1;
-                    const __nv_bfloat16 *m1 =
-                        op.mask.s1 + (((size_t)seg.b * (op.H >> up) + (y >> up)) * (op.W >> up) + (x >> up)) * op.mask.c1;
-                    const __nv_bfloat16 *m2 = op.mask.s2 ? op.mask.s2 + m * op.mask.c2 - op.mask.c1 : m1;
+                    if (NQ == 1 || y == seg.ya) {
+                        load_mask(x, y, mk);
+                    } else {
 #pragma unroll
-                    for (int k = 0; k < 2 * NQ; ++k) {
-                        const int c0 = (k >> 1) * 16 * TM_EPI + grp * 16 + (k & 1) * 8;
-                        if (c0 < op.ncols)
-                            mk[k] = __ldg(reinterpret_cast<const uint4 *>((c0 < op.mask.c1 ? m1 : m2) + c0));
+                        for (int k = 0; k < NQ; ++k)
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) mk[k][i] = next[k][i];
                     }
+                    if (NQ > 1 && y + 1 < seg.yb) load_mask(x, y + 1, next);
                 }
                 if (!(ok = mbar_wait_warp(&acc_full[n % ROLL_ACC], (uint32_t)((n / ROLL_ACC) & 1), spin))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -242,42 +271,38 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
                     if (c16 >= op.ncols) break;
                     float v[16];
                     tmem_ld16(tacc + (uint32_t)c16, v);
+                    if (op.bias) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int c0 = c16 + 8 * h;
-                        if (op.store_cols && c0 >= op.store_cols) break;
-                        float o[8];
-                        float4 ba = make_float4(0.f, 0.f, 0.f, 0.f), bb = ba;
-                        if (op.bias) {
-                            ba = __ldg(reinterpret_cast<const float4 *>(op.bias + c0));
-                            bb = __ldg(reinterpret_cast<const float4 *>(op.bias + c0 + 4));
+                        for (int i = 0; i < 16; i += 4) {
+                            const float4 b4 = __ldg(reinterpret_cast<const float4 *>(op.bias + c16 + i));
+                            v[i] += b4.x; v[i + 1] += b4.y; v[i + 2] += b4.z; v[i + 3] += b4.w;
                         }
-                        const float bs[8] = {ba.x, ba.y, ba.z, ba.w, bb.x, bb.y, bb.z, bb.w};
+                    }
+                    if (op.relu)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
+                    if (op.mask.s1)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const uint32_t w = mk[g][i >> 1];
+                            const float f = __uint_as_float((i & 1) ? (w & 0xffff0000u) : (w << 16));
+                            if (!(f > 0.f)) v[i] = 0.f;
+                        }
+                    if (op.out_f32) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 4) {
+                            if (op.store_cols && c16 + i >= op.store_cols) break;
+                            *reinterpret_cast<float4 *>((float *)op.out + m * op.Nout + c16 + i) =
+                                make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                        }
+                    } else {
+                        uint32_t o[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            const float u = v[8 * h + i] + bs[i];
-                            o[i] = op.relu ? fmaxf(u, 0.f) : u;
+                            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                            o[i] = *reinterpret_cast<const uint32_t *>(&h);
                         }
-                        if (op.mask.s1) {
-                            const uint4 mv = mk[2 * g + h];
-                            const uint32_t w4[4] = {mv.x, mv.y, mv.z, mv.w};
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                const float f = __uint_as_float((i & 1) ? (w4[i >> 1] & 0xffff0000u) : (w4[i >> 1] << 16));
-                                if (!(f > 0.f)) o[i] = 0.f;
-                            }
-                        }
-                        if (op.out_f32) {
-                            float4 *d = reinterpret_cast<float4 *>((float *)op.out + m * op.Nout + c0);
-                            d[0] = make_float4(o[0], o[1], o[2], o[3]);
-                            d[1] = make_float4(o[4], o[5], o[6], o[7]);
-                        } else {
-                            __align__(16) __nv_bfloat162 p[4];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-                            *reinterpret_cast<uint4 *>((__nv_bfloat16 *)op.out + m * op.Nout + c0) =
-                                *reinterpret_cast<const uint4 *>(p);
-                        }
+                        st32((__nv_bfloat16 *)op.out + m * op.Nout + c16, o);
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
