@@ -172,7 +172,7 @@ struct TmaBase {
     uint32_t res_bytes;         // operand bytes copied once per CTA and kept (0: none)
     uint32_t acc_cols;          // TMEM columns of one accumulator (32..512, a power of two)
     int nbuf;                   // accumulators: 2 (epilogue of tile j overlaps tile j+1) or 1
-    int ncols;                  // accumulator columns the epilogue stores (multiple of 8)
+    int ncols;                  // accumulator columns the epilogue stores (multiple of 16)
     int cps;                    // CTAs per SM (tma_fit)
 };
 
@@ -330,14 +330,16 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
             op.k_range(t, k0, k1);
             const auto R = op.row(row, t);  // per-row state, once per tile
             if (k1 > k0) {
-                for (int c0 = grp * 8; c0 < op.ncols; c0 += 8 * TM_EPI) {
-                    float v[8];
-                    tmem_ld8(tmem + (uint32_t)buf * cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+                for (int c0 = grp * 16; c0 < op.ncols; c0 += 16 * TM_EPI) {
+                    float v[16];
+                    tmem_ld16(tmem + (uint32_t)buf * cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
                     op.store_row(R, c0, v, t);
                 }
             } else {
-                const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                for (int c0 = grp * 8; c0 < op.ncols; c0 += 8 * TM_EPI) op.store_row(R, c0, z, t);
+                for (int c0 = grp * 16; c0 < op.ncols; c0 += 16 * TM_EPI) {
+                    float z[16] = {};
+                    op.store_row(R, c0, z, t);
+                }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(&acc_empty[buf]);
@@ -596,14 +598,13 @@ struct WgradTma : TmaBase {
         const int r = (int)t.x * BM + row;
         if (r > R) return;
         const int n = (int)t.y * bn + col;
-        float4 *d = reinterpret_cast<float4 *>(part + ((size_t)t.z * (R + 1) + r) * Nout + n);
-        d[0] = make_float4(v[0], v[1], v[2], v[3]);
-        d[1] = make_float4(v[4], v[5], v[6], v[7]);
+        st32(part + ((size_t)t.z * (R + 1) + r) * Nout + n, v);
     }
     struct Row { int r; };
     __device__ Row row(int r, const uint3 &) const { return Row{r}; }
     __device__ void store_row(const Row &R, int col, const float *v, const uint3 &t) const {
         store(R.r, col, v, t);
+        store(R.r, col + 8, v + 8, t);
     }
 };
 
@@ -658,6 +659,7 @@ struct GemmTma : TmaBase {
     __device__ Row row(int r, const uint3 &) const { return Row{r}; }
     __device__ void store_row(const Row &R, int col, const float *v, const uint3 &t) const {
         store(R.r, col, v, t);
+        store(R.r, col + 8, v + 8, t);
     }
 };
 
@@ -723,7 +725,7 @@ int launch_tma(const Op &op, dim3 grid, int *err, cudaStream_t stream, long long
         return kb::set_error(KB_ERR_ARG, "umma_tma_k: stage of %u bytes with %u resident bytes too large",
                              stage, op.res_bytes);
     if (op.nbuf < 1 || op.nbuf > 2 || (uint32_t)cps * op.nbuf * op.acc_cols > 512u || op.acc_cols < 32u ||
-        (op.acc_cols & (op.acc_cols - 1u)) || op.ncols > (int)op.acc_cols || op.ncols % 8)
+        (op.acc_cols & (op.acc_cols - 1u)) || op.ncols > (int)op.acc_cols || op.ncols % 16)
         return kb::set_error(KB_ERR_ARG, "umma_tma_k: accumulator shape %u x %d (store %d) invalid",
                              op.acc_cols, op.nbuf, op.ncols);
     const long long ntiles = (long long)grid.x * grid.y * grid.z;
