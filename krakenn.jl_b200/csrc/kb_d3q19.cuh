@@ -225,7 +225,8 @@ struct LinkTable3 {
 
 // One side stream and a fork / join event pair per device, created on first
 // use and kept for the life of the process: the cut-node kernel of a
-// cut-link step runs there, beside the kernel that updates the other nodes.
+// deviation-storage cut-link step runs there, beside the kernel that updates
+// the other nodes.
 // Null when the current device has none (the caller then uses its stream).
 struct SideStream {
     cudaStream_t side = nullptr;
