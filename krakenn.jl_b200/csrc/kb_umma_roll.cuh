@@ -297,15 +297,21 @@ __global__ void __launch_bounds__(TM_THREADS, NQ == 1 ? 4 : (NQ == 2 ? 2 : 1))
 // 64-pixel steps, numbered down the rows of each 64-pixel column, and keeps the
 // gradient rows r = tap C + c of its chunks (and the bias row) in TMEM.  A ring
 // stage holds the strips of input row t (one per chunk: pixels x-1 .. x+sr-2,
-// box ea x sr, MN-major, swizzle 2ea) and the output gradient of row t - 1 (nb
-// blocks of eb channels x 64 pixels); the step of output row t - 1 reads the
-// strips of rows t - 2, t - 1 and t from the last three stages, so an input row
-// is copied once, not once per kernel row (17 -> 9 KB per step at 32 channels,
-// and four or five stages where two fitted).  M-tile m = (dy, chunk, h) reads
-// its strip with the blocks one row apart (LBO = 2ea bytes): block j is the
-// strip shifted by j pixels, i.e. tap dx = 2h - 1 + j (blocks of taps beyond +1
-// are computed and not stored).  The bias M-tile reads the resident `ones` rows
-// (1 in channel 0).  Accumulator m holds columns m bn .. m bn + bn - 1.
+// box ea x sr, MN-major, swizzle 2ea) and the output gradient of row t + 1 (nb
+// blocks of eb channels x 64 pixels); the step of input row t multiplies its
+// strips with the output gradients of rows t - 1, t and t + 1 (kernel rows 2, 1
+// and 0) from the last three stages, so a row of either is copied once, not once
+// per kernel row (17 -> 9 KB per step at 32 channels, and four or five stages
+// where two fitted).  The three output gradients are one operand of N = 3 bn
+// (its blocks lie a stage apart; two MMAs where the ring wraps, and on the first
+// rows, where a kernel row starts from 0 beside one that adds): with an MMA per
+// kernel row each read the 4 KB strip again, which bounds an MMA of N = 32 (32
+// channels 51 -> 41 us, 96 -> 32 channels 130 -> 94, the gradient 2069 -> 2011).
+// An M-tile (chunk, h) reads its strip with the blocks one row apart (LBO = 2ea
+// bytes): block j is the strip shifted by j pixels, i.e. tap dx = 2h - 1 + j
+// (blocks of taps beyond +1 are computed and not stored).  The bias M-tile reads
+// the resident `ones` rows (1 in channel 0).  Columns [(3 (chunk mtp + h) + 2 -
+// kernel row) bn, + bn) hold a tile's kernel row, the last bn the bias.
 // 64-channel chunks take this form too, with one CTA per SM: per-tap boxes
 // (WgradTma) copy 120 KB per step there, this form 17 KB.  The whole gradient
 // of the batch-16 256^2 network: 2382 -> 2340 us.
@@ -326,8 +332,8 @@ struct WgradRoll {
             if (row != 0 || t.x != 0) return;
             r = R;
         } else {
-            const int st = mtp == 2 ? (m >> 1) : m, h = m - st * mtp;
-            const int dyi = st / cpt, ci = (int)t.x * cpt + st - dyi * cpt;
+            const int st = m / 3, dyi = 2 - (m - 3 * st);
+            const int cl = mtp == 2 ? (st >> 1) : st, h = st - cl * mtp, ci = (int)t.x * cpt + cl;
             const int j = row >> ea_shift, c = row & (ea - 1);
             const int dx = 2 * h - 1 + j;
             if (dx > 1) return;
@@ -400,15 +406,15 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
                 if (g >= nstages && !(ok = mbar_wait_warp(&empty[s], par ^ 1u, spin))) break;
                 if (elect_one()) {
                     const uint32_t bar = smem_u32(&full[s]), sa = base + (uint32_t)s * stage_bytes;
-                    expect_tx(bar, txs + (t > ya ? txd : 0u));
+                    expect_tx(bar, txs + (t + 1 < yb ? txd : 0u));
                     for (int ci = 0, c = cg; ci < op.cpt; ++ci, c += op.ea) {
                         const uint32_t dst = sa + (uint32_t)ci * op.strip_bytes;
                         if (c < op.c1) tma4(dst, &op.x1, c, x0 - 1, t, b, bar);
                         else tma4(dst, &op.x2, c - op.c1, x0 - 1, t, b, bar);
                     }
-                    if (t > ya)
+                    if (t + 1 < yb)
                         for (int j = 0; j < op.nb; ++j)
-                            tma4(sa + dyo + (uint32_t)(j * 128 * op.eb), &op.dy, j * op.eb, x0, t - 1, b, bar);
+                            tma4(sa + dyo + (uint32_t)(j * 128 * op.eb), &op.dy, j * op.eb, x0, t + 1, b, bar);
                 }
                 if (++s == nstages) {
                     s = 0;
@@ -428,47 +434,51 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
         if (!mbar_wait_warp(resbar, 0u, spin)) ok = false;
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
-        const uint32_t idesc = idesc_bf16(op.bn, true, true);
+        const uint32_t idesc1 = idesc_bf16(op.bn, true, true), idesc_step = idesc_bf16(2 * op.bn, true, true) - idesc1;
+        const int gmax = op.nb == 1 ? 256 / op.bn : 1;
         const uint32_t sA = 2u * (uint32_t)op.ea, sB = 2u * (uint32_t)op.eb;
         const uint32_t strip = op.strip_bytes >> 4, half = sA >> 3;  // 2 sA bytes
-        const uint32_t dyo = (uint32_t)op.cpt * op.strip_bytes;
+        const uint32_t dyo = (uint32_t)op.cpt * op.strip_bytes, lbo = op.nb == 1 ? stage_bytes : 64u * sB;
         const Desc ones = desc_sw(res, sA, 8u * sA, sA);
         int s = 0, s1 = 0, s2 = 0;  // this stage's slot and the two before
-        uint32_t par = 0, on = 0;
+        uint32_t par = 0, begun = 0;  // begun: kernel rows (bit 2 - row) and bias (bit 3) that hold a sum
         ok = mbar_wait_warp(resbar, 0u, spin);
         for (int r = r0; r < r1 && ok;) {
             const int col = r / op.H, ya = r - col * op.H, yb = min(op.H, ya + (r1 - r));
             r += yb - ya;
             for (int t = ya - 1; t <= yb; ++t) {
                 if (!(ok = mbar_wait_warp(&full[s], par, spin))) break;
-                if (t > ya) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (elect_one()) {
-                        const Desc b = desc_mn(base + (uint32_t)s * stage_bytes + dyo, sB);
-                        uint32_t accm = tmem;
-                        for (int dyi = 0; dyi < 3; ++dyi) {
-                            const int slot = dyi == 0 ? s2 : (dyi == 1 ? s1 : s);
-                            const Desc a = desc_sw(base + (uint32_t)slot * stage_bytes, sA, 8u * sA, sA);
-                            uint32_t a0 = 0;
-                            for (int ci = 0; ci < op.cpt; ++ci, a0 += strip) {
-                                mma_run<BK / 16>(accm, a, a0, sA, b, 0u, sB, idesc, on);
-                                accm += (uint32_t)op.bn;
-                                if (op.mtp == 2) {
-                                    mma_run<BK / 16>(accm, a, a0 + half, sA, b, 0u, sB, idesc, on);
-                                    accm += (uint32_t)op.bn;
-                                }
-                            }
-                        }
-                        if (grp == 0) mma_run<BK / 16>(accm, ones, 0u, sA, b, 0u, sB, idesc, on);
-                        mma_commit(&empty[s2]);
-                        if (t == yb) {
-                            mma_commit(&empty[s1]);
-                            mma_commit(&empty[s]);
-                        }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                // input row t meets output rows t - 1 + o, kernel row 2 - o
+                const int o0 = max(0, ya - t + 1), o1 = min(2, yb - t);
+                if (elect_one()) {
+                    const Desc a = desc_sw(base + (uint32_t)s * stage_bytes, sA, 8u * sA, sA);
+                    uint32_t was = begun;
+                    for (int o = o0; o <= o1;) {
+                        const int slot = o == 0 ? s2 : (o == 1 ? s1 : s);
+                        const uint32_t on = was >> o & 1u;
+                        int run = 1;
+                        while (o + run <= o1 && run < gmax && slot + run < nstages && (was >> (o + run) & 1u) == on) ++run;
+                        const Desc b = desc_sw(base + (uint32_t)slot * stage_bytes + dyo, lbo, 8u * sB, sB);
+                        const uint32_t idesc = idesc1 + (uint32_t)(run - 1) * idesc_step;
+                        uint32_t accm = tmem + (uint32_t)(o * op.bn), a0 = 0;
+                        for (int ci = 0; ci < op.cpt; ++ci, a0 += strip)
+                            for (int h = 0; h < op.mtp; ++h, accm += (uint32_t)(3 * op.bn))
+                                mma_run<BK / 16>(accm, a, a0 + (uint32_t)h * half, sA, b, 0u, sB, idesc, on);
+                        o += run;
                     }
-                    __syncwarp();
-                    on = 1u;
+                    if (grp == 0 && t + 1 < yb)
+                        mma_run<BK / 16>(tmem + (uint32_t)(op.nmt * op.bn), ones, 0u, sA,
+                                         desc_mn(base + (uint32_t)s * stage_bytes + dyo, sB), 0u, sB, idesc1, was >> 3);
+                    if (t > ya) mma_commit(&empty[s2]);
+                    if (t == yb) {
+                        mma_commit(&empty[s1]);
+                        mma_commit(&empty[s]);
+                    }
                 }
+                __syncwarp();
+                for (int o = o0; o <= o1; ++o) begun |= 1u << o;
+                if (t + 1 < yb) begun |= 8u;
                 s2 = s1;
                 s1 = s;
                 if (++s == nstages) {
