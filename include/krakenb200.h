@@ -590,8 +590,13 @@ int kb_batch_populations(kb_batch *b, int c, void **f, int *dtype, void *stream)
  * replay it with kb_graph_launch.  This is the device-side form of
  * persistent_fused_bgk! / persistent_aa_bgk! (src/kernels/persistent_bgk_2d.jl:
  * 17-56), which queue Nt launches from the host.  Calls that synchronise or
- * allocate (kb_mass, kb_residual, kb_batch_create ...) cannot be captured. */
+ * allocate (kb_mass, kb_residual, kb_batch_create ...) cannot be captured.
+ * Whatever any thread queues on `stream` in between is captured with them:
+ * kb_stream_create makes a non-blocking stream of the current device that
+ * nobody else holds. */
 typedef struct kb_graph kb_graph;
+int kb_stream_create(void **stream);
+int kb_stream_destroy(void *stream);
 int kb_graph_begin(void *stream);
 int kb_graph_end(void *stream, kb_graph **out);
 int kb_graph_launch(kb_graph *g, void *stream);

@@ -117,6 +117,8 @@ SIGNATURES: dict[str, list] = {
                       C.POINTER(C.c_float), C.POINTER(C.c_float), _vp],
     "kb_batch_autotune": [_vp, _i, C.POINTER(_i), C.POINTER(_i), _dp, _dp, _vp],
     "kb_batch_populations": [_vp, _i, C.POINTER(_vp), C.POINTER(_i), _vp],
+    "kb_stream_create": [C.POINTER(_vp)],
+    "kb_stream_destroy": [_vp],
     "kb_graph_begin": [_vp],
     "kb_graph_end": [_vp, C.POINTER(_vp)],
     "kb_graph_launch": [_vp, _vp],

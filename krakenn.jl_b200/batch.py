@@ -127,22 +127,27 @@ class CavityBatch:
 
 
 class Graph:
-    """Capture library calls issued on a side stream, then replay them."""
+    """Capture library calls issued on a stream of its own, then replay them.
+    The stream is not one of torch's pool, which hands the same 32 streams out
+    in turn: another thread's work queued on a pool stream while a graph
+    captures on it would be captured instead of run."""
 
     def __init__(self):
         self._g = C.c_void_p()
-        self.stream = torch.cuda.Stream()
+        self._s = C.c_void_p()
+        call("kb_stream_create", C.byref(self._s))
+        self.stream = torch.cuda.ExternalStream(self._s.value)
 
     def __enter__(self):
         self.stream.wait_stream(torch.cuda.current_stream())
+        call("kb_graph_begin", self._s)
         self._ctx = torch.cuda.stream(self.stream)
         self._ctx.__enter__()
-        call("kb_graph_begin", C.c_void_p(self.stream.cuda_stream))
         return self
 
     def __exit__(self, *exc):
         try:
-            call("kb_graph_end", C.c_void_p(self.stream.cuda_stream), C.byref(self._g))
+            call("kb_graph_end", self._s, C.byref(self._g))
         finally:
             self._ctx.__exit__(*exc)
         return False
@@ -154,6 +159,9 @@ class Graph:
         if self._g:
             call("kb_graph_destroy", self._g)
             self._g = C.c_void_p()
+        if self._s:
+            call("kb_stream_destroy", self._s)
+            self._s = C.c_void_p()
 
     def __del__(self):
         try:

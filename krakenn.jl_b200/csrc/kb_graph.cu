@@ -43,6 +43,22 @@ __global__ void wait_selftest_k(unsigned *word, long long limit, int *err, long 
 
 extern "C" {
 
+int kb_stream_create(void **stream) {
+    KB_REQUIRE(stream, "kb_stream_create: null pointer");
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return kb::set_error(KB_ERR_CUDA, "kb_stream_create: %s", cudaGetErrorString(e));
+    *stream = s;
+    return KB_OK;
+}
+
+int kb_stream_destroy(void *stream) {
+    if (!stream) return KB_OK;
+    cudaError_t e = cudaStreamDestroy(kb::as_stream(stream));
+    if (e != cudaSuccess) return kb::set_error(KB_ERR_CUDA, "kb_stream_destroy: %s", cudaGetErrorString(e));
+    return KB_OK;
+}
+
 int kb_graph_begin(void *stream) {
     KB_REQUIRE(stream, "kb_graph_begin: capture needs a non-default stream");
     cudaError_t e = cudaStreamBeginCapture(kb::as_stream(stream), cudaStreamCaptureModeThreadLocal);
