@@ -607,6 +607,10 @@ int kb_graph_destroy(kb_graph *g);
  * polls it gives up, sets the error flag and returns.  *timed_out = 1 and
  * KB_ERR_TIMEOUT is the expected result.  No reference counterpart. */
 int kb_selftest_bounded_wait(long long limit, int *timed_out, void *stream);
+/* A 64-step kb_cavity_run_2d of 16 blocks on buffers of its own whose waits
+ * give up after `limit` rounds of polls (-1: at the first miss; at most the
+ * 2^21 of kb_cavity_run_2d): KB_ERR_TIMEOUT and *gave_up = 1 if one did. */
+int kb_selftest_cavity_run(long long limit, int *gave_up, void *stream);
 
 /* ------------------------------------------------- precision utilities -- */
 

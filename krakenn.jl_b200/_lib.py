@@ -124,6 +124,7 @@ SIGNATURES: dict[str, list] = {
     "kb_graph_launch": [_vp, _vp],
     "kb_graph_destroy": [_vp],
     "kb_selftest_bounded_wait": [C.c_longlong, C.POINTER(_i), _vp],
+    "kb_selftest_cavity_run": [C.c_longlong, C.POINTER(_i), _vp],
     "kb_convert_populations": [_vp, _i, _cvp, _i, _i, _sz, _vp],
     "kb_set_stochastic_seed": [C.c_uint, _vp],
     "kb_get_stochastic_seed": [C.POINTER(C.c_uint), _vp],

@@ -1672,6 +1672,38 @@ int kb_cavity_run_2d(void *f_0, void *f_1, void *rho, void *ux, void *uy, const 
         if (rc) return rc);
 }
 
+int kb_selftest_cavity_run(long long limit, int *gave_up, void *stream) {
+    const char *what = "kb_selftest_cavity_run";
+    KB_REQUIRE(gave_up, "%s: null pointer", what);
+    KB_REQUIRE(limit >= -1 && limit <= RES_SPIN, "%s: limit out of range", what);
+    constexpr int Nx = 4 * RES_W, Ny = 4 * RES_H, n = Nx * Ny;  // 16 tiles
+    const size_t ws = cavity_run_bytes<float, false>(Nx, Ny), pops = (size_t)9 * n * sizeof(float);
+    KB_REQUIRE(ws > 0, "%s: no cooperative launch on this device", what);
+    cudaStream_t s = kb::as_stream(stream);
+    char *buf = nullptr;
+    cudaError_t e = cudaMallocAsync((void **)&buf, ws + 2 * pops + 3 * n * sizeof(float), s);
+    if (e != cudaSuccess) return kb::set_error(KB_ERR_NOMEM, "%s: %s", what, cudaGetErrorString(e));
+    e = cudaMemsetAsync(buf + ws, 0, pops, s);
+    CavityRun<float> R = {};
+    R.f0 = (float *)(buf + ws);
+    R.f1 = R.f0 + 9 * n;
+    R.rho = R.f1 + 9 * n;
+    R.ux = R.rho + n;
+    R.uy = R.ux + n;
+    R.Nx = Nx; R.Ny = Ny; R.nsteps = 64;
+    R.omega = 1.0f;
+    int rc = KB_OK, flag = 0;
+    if (e == cudaSuccess) rc = cavity_run<float, false>(what, R, buf, ws, s, limit);
+    if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(&flag, buf, sizeof(int), cudaMemcpyDeviceToHost, s);
+    cudaFreeAsync(buf, s);
+    if (e == cudaSuccess && !rc) e = cudaStreamSynchronize(s);
+    if (rc) return rc;
+    if (e != cudaSuccess) return kb::set_error(KB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    *gave_up = flag;
+    return flag ? kb::set_error(KB_ERR_TIMEOUT, "%s: a wait between blocks gave up after %lld rounds", what, limit)
+                : KB_OK;
+}
+
 int kb_cavity_mrt_step_2d(void *f_out, const void *f_in, void *rho, void *ux, void *uy,
                           const uint8_t *is_solid, int Nx, int Ny, double nu, double s_e,
                           double s_eps, double s_q, double u_lid, int dtype, void *stream) {

@@ -24,7 +24,8 @@
 // Packets are 64-bit words, 32 bits of value and 32 of step number, so a word
 // is either old or new.  Blocks wait for one another, so the launch is
 // cooperative; a wait that exceeds its limit sets the error flag, and its
-// thread and those that see the flag wait no more.
+// thread and those that see the flag wait no more: every thread still takes
+// all its steps, so the launch ends, with void results.
 #pragma once
 #include "kb_common.cuh"
 
@@ -189,8 +190,12 @@ size_t cavity_run_bytes(int Nx, int Ny) {
     return RES_HEADER + (size_t)2 * 8 * Nx * Ny * sizeof(Packet<T>);
 }
 
+// Rounds of polls in one step before a wait gives up, about a microsecond each.
+constexpr long long RES_SPIN = 1ll << 21;
+
 template <typename T, bool MOVING>
-int cavity_run(const char *what, CavityRun<T> R, void *workspace, size_t bytes, cudaStream_t s) {
+int cavity_run(const char *what, CavityRun<T> R, void *workspace, size_t bytes, cudaStream_t s,
+               long long spin = RES_SPIN) {
     const size_t need = cavity_run_bytes<T, MOVING>(R.Nx, R.Ny);
     KB_REQUIRE(need > 0, "%s: a %d x %d grid is not resident on the device at once", what, R.Nx, R.Ny);
     KB_REQUIRE(bytes >= need, "%s: workspace of %zu bytes, %zu needed", what, bytes, need);
@@ -198,7 +203,7 @@ int cavity_run(const char *what, CavityRun<T> R, void *workspace, size_t bytes, 
     const dim3 grid = cavity_run_grid(R.Nx, R.Ny, &R.tw);
     R.err = (int *)workspace;
     R.packets = (unsigned char *)workspace + RES_HEADER;
-    R.spin = 1ll << 21;  // rounds of polls in one step, about a microsecond each
+    R.spin = spin;
     void *args[] = {&R};
     if (cudaLaunchCooperativeKernel((void *)cavity_run_k<T, MOVING>, grid, dim3(RES_W, RES_H), args, 0, s) !=
         cudaSuccess)

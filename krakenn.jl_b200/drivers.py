@@ -115,7 +115,9 @@ def run_cavity_2d(config: LBMConfig, backend="b200", T=torch.float64, fused=True
     lid="moving_wall": half-way bounce-back on all four walls with the
     moving-wall link rule on the lid (kb_cavity_movingwall_step_2d).
     Without on_step, a grid that is resident on the device at once (about
-    256^2) runs all its steps in one launch (kb_cavity_run_2d, same bits).
+    256^2) runs all its steps in one launch (kb_cavity_run_2d, same bits); a
+    launch whose blocks gave up a wait for one another raises RuntimeError, and
+    the populations and moments in `state` are then void.
     on_step(step, fields): called after every step with the device moment
     fields (for example an output.StepOutput)."""
     _require_backend(backend)

@@ -59,3 +59,36 @@ def test_grids_that_do_not_fit_are_refused(cuda, pkg):
     sm = [t[:8, :8].contiguous() for t in m]
     with pytest.raises(pkg.KrakenArgumentError):  # workspace too small
         pkg.ops.cavity_run_2d_(*small, *sm, None, 8, 8, 1.0, 0.1, False, 4, ws[:16])
+
+
+def test_a_wait_that_gives_up_is_reported(cuda, pkg, monkeypatch):
+    """Blocks whose first missed poll gives up set the flag and end the launch,
+    and the context stays usable; the driver raises on the flag."""
+    import ctypes as C
+    from importlib import import_module
+    lib = import_module(pkg.__name__ + "._lib")
+    drivers = import_module(pkg.__name__ + ".drivers")
+    flag = C.c_int(-1)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    lib.call("kb_selftest_cavity_run", C.c_longlong(1 << 21), C.byref(flag), stream)
+    assert flag.value == 0
+    with pytest.raises(lib.KrakenError) as e:
+        lib.call("kb_selftest_cavity_run", C.c_longlong(-1), C.byref(flag), stream)
+    assert e.value.code == lib.KB_ERR_TIMEOUT and flag.value == 1
+    for bad in (-2, (1 << 21) + 1):
+        with pytest.raises(lib.KrakenArgumentError):
+            lib.call("kb_selftest_cavity_run", C.c_longlong(bad), C.byref(flag), stream)
+
+    cfg = pkg.LBMConfig.d2q9(70, 6, 0.05, 0.1, 40)
+    want = pkg.run_cavity_2d(cfg)
+    run = drivers.ops.cavity_run_2d_
+
+    def gave_up(*a):
+        run(*a)
+        a[-1][0] = 1
+
+    with monkeypatch.context() as m:
+        m.setattr(drivers.ops, "cavity_run_2d_", gave_up)
+        with pytest.raises(RuntimeError, match="gave up"):
+            pkg.run_cavity_2d(cfg)
+    assert (pkg.run_cavity_2d(cfg)["ux"] == want["ux"]).all()
