@@ -613,12 +613,10 @@ int conv_strip(kb::umma::ConvStrip &c, const bf16 *x1, int c1, const bf16 *x2, i
     c.nck = C / e;
     c.strip_bytes = round1k((uint32_t)((BM + 2) * 2 * e));
     c.acc_cols = tmem_cols(bn);
-    c.nbuf = 2;
     c.ncols = bn;
     c.tx = (uint32_t)((BM + 2) * 2 * e + 3 * bn * 2 * e);
     c.a_bytes = c.strip_bytes;
     c.b_bytes = round1k((uint32_t)(3 * bn * 2 * e));
-    c.res_bytes = 0;
     c.cps = tma_fit(c);
     return 0;
 }
@@ -666,7 +664,6 @@ bool conv_strip_fits(int C, int e, int bn, int W) {
     t.a_bytes = r.strip_bytes;
     t.b_bytes = round1k((uint32_t)(3 * bn * 2 * e));
     t.acc_cols = tmem_cols(bn);
-    t.nbuf = 2;
     return r.cps > 0 || tma_fit(t) > 0;
 }
 
@@ -730,9 +727,7 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         c.nck = cin / ef;
         c.a_bytes = round1k((uint32_t)(BM * 2 * ef));
         c.b_bytes = round1k((uint32_t)(l.bn_f * 2 * ef));
-        c.res_bytes = 0;
         c.acc_cols = tmem_cols(l.bn_f);
-        c.nbuf = 2;
         c.ncols = l.bn_f;
         c.cps = tma_fit(c);
         c.tx = (uint32_t)(BM * 2 * ef + l.bn_f * 2 * ef);
@@ -781,9 +776,7 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         c.nck = l.cout / ed;
         c.a_bytes = round1k((uint32_t)(BM * 2 * ed));
         c.b_bytes = round1k((uint32_t)(l.bn_d * 2 * ed));
-        c.res_bytes = 0;
         c.acc_cols = tmem_cols(l.bn_d);
-        c.nbuf = 2;
         c.ncols = l.bn_d;
         c.cps = tma_fit(c);
         c.tx = (uint32_t)(BM * 2 * ed + l.bn_d * 2 * ed);
@@ -869,9 +862,7 @@ int prepare_tma(kb_surrogate *s, int i, int n) {
         w.nb = l.bn_w / eb;
         w.a_bytes = BM * BK * 2;
         w.b_bytes = round1k((uint32_t)(l.bn_w * BK * 2));
-        w.res_bytes = 0;
         w.acc_cols = tmem_cols(l.bn_w);
-        w.nbuf = 2;
         w.ncols = l.bn_w;
         w.cps = tma_fit(w);
         p.w = w.cps ? 1 : 0;

@@ -3,10 +3,10 @@
 //
 // cps persistent CTAs per SM (64 + 128 TM_EPI threads each) loop over the
 // tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... of the grid `tiles` (x
-// fastest).  One warp issues at most one tcgen05.mma about every 180 cycles
-// whatever N is, so an N = 32 tile reaches 1/8 of the tensor rate from one
-// issuer; several CTAs per SM, each with its own ring, MMA lane and share of
-// TMEM, multiply the issue rate.  In each CTA:
+// fastest).  One warp issues a tcgen05.mma about every 60 cycles (every 180
+// with the loop on one lane) whatever N is, so narrow tiles do not fill the
+// tensor cores from one issuer; several CTAs per SM, each with its own ring,
+// MMA warp and share of TMEM, multiply the issue rate.  In each CTA:
 //   warp 0    producer: waits for a free ring stage (`empty`), posts the
 //             stage's byte count on its `full` barrier and issues the step's
 //             cp.async.bulk.tensor copies, one per operand box;
@@ -20,7 +20,7 @@
 //             with an elected lane 2491, with the stepped descriptors 2482;
 //   warps 2.. epilogue, TM_EPI warps per TMEM lane quarter: warp w reads
 //             TMEM lanes 32(w%4)..+31 (tile rows) of the finished
-//             accumulator, every TM_EPI-th group of 8 columns, calls op.store
+//             accumulator, every TM_EPI-th group of 16 columns, calls op.store
 //             and arrives on `acc_empty`, so the epilogue of tile j overlaps
 //             the MMAs of tile j+1.  Several warps per quarter keep several
 //             TMEM-load / store chains of a tile in flight.
@@ -169,9 +169,7 @@ struct TileCursor {
 // Fields every operation carries (set on the host).
 struct TmaBase {
     uint32_t a_bytes, b_bytes;  // operand bytes of one ring stage (multiples of 1024)
-    uint32_t res_bytes;         // operand bytes copied once per CTA and kept (0: none)
-    uint32_t acc_cols;          // TMEM columns of one accumulator (32..512, a power of two)
-    int nbuf;                   // accumulators: 2 (epilogue of tile j overlaps tile j+1) or 1
+    uint32_t acc_cols;          // TMEM columns of each of the two accumulators (32..256, a power of two)
     int ncols;                  // accumulator columns the epilogue stores (multiple of 16)
     int cps;                    // CTAs per SM (tma_fit)
 };
@@ -180,12 +178,11 @@ struct TmaBase {
 //   static constexpr bool A_MN, B_MN;
 //   __device__ uint32_t step_tx(const uint3 &t)    bytes the copies of one step of tile t bring
 //   __device__ void prefetch()                     prefetch the tensor maps
-//   __device__ void issue_res(uint32_t res, uint32_t bar)   copies of the resident operand
 //   struct Cursor; __device__ Cursor begin(const uint3 &t, int k0)   state of step k0 of tile t
 //   __device__ void issue(Cursor &c, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead)
 //                                                  the lead lane's copies of the cursor's step; advance it
-//   __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t res, int kt, int k0,
-//                       const uint3 &t, uint32_t idesc)   the MMAs of step kt of tile t
+//   __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, int kt, int k0, uint32_t idesc)
+//                                                  the MMAs of step kt of a tile that starts with step k0
 template <class Op>
 __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
     umma_tma_k(const __grid_constant__ Op op, const uint3 tiles, const int nstages,
@@ -194,21 +191,17 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     const uint32_t stage_bytes = op.a_bytes + op.b_bytes;
-    const uint32_t res = base + (uint32_t)nstages * stage_bytes;  // resident operand
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw + (base - raw) + (size_t)nstages * stage_bytes +
-                                                  op.res_bytes);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw + (base - raw) + (size_t)nstages * stage_bytes);
     uint64_t *empty = full + nstages;
     uint64_t *acc_full = empty + nstages, *acc_empty = acc_full + 2, *drain = acc_empty + 2;
-    uint64_t *resbar = drain + 1;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(resbar + 1);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t cols = op.acc_cols;
-    const int nbuf = op.nbuf;
     const int ntiles = (int)(tiles.x * tiles.y * tiles.z);  // < 2^31 (checked by launch_tma)
 
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)nbuf * cols));
+                     ::"r"(smem_u32(tmem_slot)), "r"(2u * cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
@@ -221,7 +214,6 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
             mbar_init(&acc_empty[i], 128 * TM_EPI);
         }
         mbar_init(drain, 1);
-        mbar_init(resbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -237,10 +229,6 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
         // ---------------------------------------------------------- producer
         {
             if (elect_one()) op.prefetch();
-            if (op.res_bytes && elect_one()) {
-                expect_tx(smem_u32(resbar), op.res_bytes);
-                op.issue_res(res, smem_u32(resbar));
-            }
             long long g = 0;
             int s = 0;
             uint32_t par = 0;
@@ -274,7 +262,6 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
                 --s;
                 if (!mbar_wait_warp(&full[s], par, spin)) ok = false;
             }
-            if (op.res_bytes && !mbar_wait_warp(resbar, 0u, spin)) ok = false;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -283,10 +270,9 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
             const uint32_t idesc = idesc_bf16(op.bn, Op::A_MN, Op::B_MN);
             int s = 0, j = 0;
             uint32_t par = 0;
-            if (op.res_bytes) ok = mbar_wait_warp(resbar, 0u, spin);
             TileCursor tc(tiles);
             for (int T = blockIdx.x; T < ntiles && ok; T += gridDim.x, ++j) {
-                const int buf = nbuf == 2 ? (j & 1) : 0, use = nbuf == 2 ? (j >> 1) : j;
+                const int buf = j & 1, use = j >> 1;
                 if (use >= 1 && !(ok = mbar_wait_warp(&acc_empty[buf], (uint32_t)((use - 1) & 1), spin))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint3 t = tc.at(T);
@@ -298,7 +284,7 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = base + (uint32_t)s * stage_bytes;
                     if (elect_one()) {
-                        op.mma(acc, sa, sa + op.a_bytes, res, kt, k0, t, idesc);
+                        op.mma(acc, sa, sa + op.a_bytes, kt, k0, idesc);
                         mma_commit(&empty[s]);
                     }
                     __syncwarp();
@@ -322,7 +308,7 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
         int j = 0;
         TileCursor tc(tiles);
         for (int T = blockIdx.x; T < ntiles && ok; T += gridDim.x, ++j) {
-            const int buf = nbuf == 2 ? (j & 1) : 0, use = nbuf == 2 ? (j >> 1) : j;
+            const int buf = j & 1, use = j >> 1;
             if (!(ok = mbar_wait(&acc_full[buf], (uint32_t)(use & 1), spin))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint3 t = tc.at(T);
@@ -350,7 +336,7 @@ __global__ void __launch_bounds__(TM_THREADS, TM_MAX_CPS)
     __syncthreads();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"((uint32_t)nbuf * cols));
+                     "r"(2u * cols));
 }
 
 // Ring stages that fit beside a resident operand of `res_bytes` with cps
@@ -368,8 +354,8 @@ inline size_t tma_smem_bytes(int nstages, uint32_t stage_bytes, uint32_t res_byt
 // accumulators fit TMEM together; 0 if not even one CTA fits.
 inline int tma_fit(const TmaBase &b) {
     for (int c = TM_MAX_CPS; c >= 1; --c)
-        if (tma_stages(b.a_bytes + b.b_bytes, b.res_bytes, c) >= 2 &&
-            (uint32_t)c * (uint32_t)b.nbuf * b.acc_cols <= 512u && c * TM_THREADS <= 2048)
+        if (tma_stages(b.a_bytes + b.b_bytes, 0u, c) >= 2 && (uint32_t)c * 2u * b.acc_cols <= 512u &&
+            c * TM_THREADS <= 2048)
             return c;
     return 0;
 }
@@ -417,8 +403,11 @@ struct ConvTma : ConvStore, TmaBase {
         return u;
     }
     __device__ void issue(Cursor &u, const uint3 &t, uint32_t sa, uint32_t sb, uint32_t bar, bool lead) const {
-        if (lead) { if (u.c < c1) tma4(sa, &x1, u.c, u.x + u.dx, u.y + u.dy, u.b, bar); else tma4(sa, &x2, u.c - c1, u.x + u.dx, u.y + u.dy, u.b, bar); }
-        if (lead) tma2(sb, &w, u.wk, (int)t.y * bn, bar);
+        if (lead) {
+            if (u.c < c1) tma4(sa, &x1, u.c, u.x + u.dx, u.y + u.dy, u.b, bar);
+            else tma4(sa, &x2, u.c - c1, u.x + u.dx, u.y + u.dy, u.b, bar);
+            tma2(sb, &w, u.wk, (int)t.y * bn, bar);
+        }
         u.wk += e;
         u.c += e;
         if (u.c == C) {
@@ -429,9 +418,7 @@ struct ConvTma : ConvStore, TmaBase {
             }
         }
     }
-    __device__ void issue_res(uint32_t, uint32_t) const {}
-    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int k0, const uint3 &,
-                        uint32_t idesc) const {
+    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, int kt, int k0, uint32_t idesc) const {
         const uint32_t s = 2u * (uint32_t)e, on = kt == k0 ? 0u : 1u;
         const Desc a = desc_k(sa, s), b = desc_k(sb, s);
         if (e == 64) mma_run<4>(acc, a, 0u, 2u, b, 0u, 2u, idesc, on);
@@ -463,7 +450,6 @@ struct ConvStrip : ConvStore, TmaBase {
         if (c1 < C) prefetch_map(&x2);
         prefetch_map(&w);
     }
-    __device__ void issue_res(uint32_t, uint32_t) const {}
     struct Cursor { int dy, ci, b, y, x; };
     __device__ Cursor begin(const uint3 &t, int) const {
         Cursor u;
@@ -486,8 +472,7 @@ struct ConvStrip : ConvStore, TmaBase {
             ++u.dy;
         }
     }
-    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int, const uint3 &,
-                        uint32_t idesc) const {
+    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, int kt, int, uint32_t idesc) const {
         if (e == 64) mma_e<4>(acc, sa, sb, kt, idesc);
         else if (e == 32) mma_e<2>(acc, sa, sb, kt, idesc);
         else mma_e<1>(acc, sa, sb, kt, idesc);
@@ -554,7 +539,10 @@ struct WgradTma : TmaBase {
             const uint32_t dst = sa + (uint32_t)(j * 128 * ea);
             if (r < R) {
                 const int dyy = tap / 3 - 1, dxx = tap % 3 - 1;
-                if (lead) { if (c < c1) tma4(dst, &x1, c, u.x + dxx, u.y + dyy, u.b, bar); else tma4(dst, &x2, c - c1, u.x + dxx, u.y + dyy, u.b, bar); }
+                if (lead) {
+                    if (c < c1) tma4(dst, &x1, c, u.x + dxx, u.y + dyy, u.b, bar);
+                    else tma4(dst, &x2, c - c1, u.x + dxx, u.y + dyy, u.b, bar);
+                }
             } else if (r == R) {
                 if (lead) tma2(dst, &ones, 0, 0, bar);
             }
@@ -587,9 +575,7 @@ struct WgradTma : TmaBase {
             }
         }
     }
-    __device__ void issue_res(uint32_t, uint32_t) const {}
-    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int k0, const uint3 &,
-                        uint32_t idesc) const {
+    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, int kt, int k0, uint32_t idesc) const {
         const uint32_t s_a = 2u * (uint32_t)ea, s_b = 2u * (uint32_t)eb;
         mma_run<BK / 16>(acc, desc_mn(sa, s_a), 0u, s_a, desc_mn(sb, s_b), 0u, s_b, idesc, kt == k0 ? 0u : 1u);
     }
@@ -642,9 +628,7 @@ struct GemmTma : TmaBase {
         }
         u.k += BK;
     }
-    __device__ void issue_res(uint32_t, uint32_t) const {}
-    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t, int kt, int k0, const uint3 &,
-                        uint32_t idesc) const {
+    __device__ void mma(uint32_t acc, uint32_t sa, uint32_t sb, int kt, int k0, uint32_t idesc) const {
         const uint32_t s_b = BMN ? 2u * (uint32_t)eb : 128u;
         const Desc a = AMN ? desc_mn(sa, 128u) : desc_k(sa, 128u), b = BMN ? desc_mn(sb, s_b) : desc_k(sb, s_b);
         mma_run<BK / 16>(acc, a, 0u, AMN ? 128u : 2u, b, 0u, BMN ? s_b : 2u, idesc, kt == k0 ? 0u : 1u);
@@ -720,20 +704,18 @@ int launch_tma(const Op &op, dim3 grid, int *err, cudaStream_t stream, long long
     }
     const uint32_t stage = op.a_bytes + op.b_bytes;
     const int cps = op.cps < 1 ? 1 : (op.cps > TM_MAX_CPS ? TM_MAX_CPS : op.cps);
-    const int ns = tma_stages(stage, op.res_bytes, cps);
-    if (ns < 2)
-        return kb::set_error(KB_ERR_ARG, "umma_tma_k: stage of %u bytes with %u resident bytes too large",
-                             stage, op.res_bytes);
-    if (op.nbuf < 1 || op.nbuf > 2 || (uint32_t)cps * op.nbuf * op.acc_cols > 512u || op.acc_cols < 32u ||
-        (op.acc_cols & (op.acc_cols - 1u)) || op.ncols > (int)op.acc_cols || op.ncols % 16)
-        return kb::set_error(KB_ERR_ARG, "umma_tma_k: accumulator shape %u x %d (store %d) invalid",
-                             op.acc_cols, op.nbuf, op.ncols);
+    const int ns = tma_stages(stage, 0u, cps);
+    if (ns < 2) return kb::set_error(KB_ERR_ARG, "umma_tma_k: stage of %u bytes too large", stage);
+    if ((uint32_t)cps * 2u * op.acc_cols > 512u || op.acc_cols < 32u || (op.acc_cols & (op.acc_cols - 1u)) ||
+        op.ncols > (int)op.acc_cols || op.ncols % 16)
+        return kb::set_error(KB_ERR_ARG, "umma_tma_k: accumulator shape %u (store %d) invalid", op.acc_cols,
+                             op.ncols);
     const long long ntiles = (long long)grid.x * grid.y * grid.z;
     if (ntiles >= (1ll << 31) - (1ll << 16))
         return kb::set_error(KB_ERR_ARG, "umma_tma_k: %lld tiles exceed the tile index range", ntiles);
     const long long slots = (long long)kb::sm_count() * cps;
     const long long ctas = ntiles < slots ? ntiles : slots;
-    umma_tma_k<Op><<<(unsigned)ctas, TM_THREADS, tma_smem_bytes(ns, stage, op.res_bytes), stream>>>(
+    umma_tma_k<Op><<<(unsigned)ctas, TM_THREADS, tma_smem_bytes(ns, stage, 0u), stream>>>(
         op, make_uint3(grid.x, grid.y, grid.z), ns, err, spin);
     return 0;
 }
