@@ -499,19 +499,17 @@ def run_rayleigh_benard_2d(Nx=128, Ny=32, Ra=2000.0, Pr=1.0, T_hot=1.0, T_cold=0
                 alpha=p["alpha"], T_hot=T_hot, T_cold=T_cold, orientation=orientation)
 
 
-def natconv_3d_initial_g(N, T_hot=1.0, T_cold=0.0):
-    """g = w_q T_init, linear in x between the half-way walls
-    (src/drivers/thermal.jl:481-490)."""
-    dT = T_hot - T_cold
-    i = np.arange(1, N + 1, dtype=np.float64)
-    T0 = np.broadcast_to(T_hot - dT * (i - 0.5) / N, (N, N, N))
-    return np.stack([L.D3Q19_W[q] * T0 for q in range(19)])
-
-
 def _natconv_3d_initial_T(N, T_hot, T_cold):
-    """The x profile of natconv_3d_initial_g, broadcast along y and z."""
+    """T_init of run_natural_convection_3d (src/drivers/thermal.jl:481-490):
+    linear in x between the half-way walls, to be broadcast along y and z."""
     i = np.arange(1, N + 1, dtype=np.float64)
     return (T_hot - (T_hot - T_cold) * (i - 0.5) / N)[None, None, :]
+
+
+def natconv_3d_initial_g(N, T_hot=1.0, T_cold=0.0):
+    """g = w_q T_init (src/drivers/thermal.jl:481-490)."""
+    T0 = np.broadcast_to(_natconv_3d_initial_T(N, T_hot, T_cold), (N, N, N))
+    return np.stack([L.D3Q19_W[q] * T0 for q in range(19)])
 
 
 def natconv_3d_parameters(N, Ra, Pr, T_hot=1.0, T_cold=0.0):
