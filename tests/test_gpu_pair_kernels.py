@@ -96,6 +96,31 @@ def test_cut_link_pairs_equal_one_node(cuda, pkg, size, periodic):
     links.close()
 
 
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_cut_links_without_planes_left(cuda, pkg, dtype):
+    """At 65535 planes the launch has none left for the cut nodes, so the link
+    code runs at every node; the dense arrays' step gives the same bits."""
+    Nx, Ny, Nz = 4, 3, 65535
+    shape = (Nz, Ny, Nx)
+    gen = torch.Generator(device=cuda).manual_seed(9)
+    rand = lambda *s: torch.rand(s, generator=gen, dtype=dtype, device=cuda)
+    w = torch.from_numpy(W19).to(cuda, dtype).view(19, 1, 1, 1)
+    fi = w * (1 + 0.1 * (rand(19, *shape) - 0.5))
+    qw = rand(19, *shape)
+    qw[rand(19, *shape) < 0.9] = 0
+    qw[0] = 0
+    uw = [0.02 * (rand(19, *shape) - 0.5) for _ in range(3)]
+    solid = (rand(*shape) < 0.15).to(torch.uint8)
+    links = pkg.libb.CutLinks(solid, qw, *uw)
+    a, b = torch.empty_like(fi), torch.empty_like(fi)
+    ma, mb = ([torch.empty(shape, dtype=dtype, device=cuda) for _ in range(4)] for _ in range(2))
+    pkg.fused_trt_libb_links_step_3d_(a, fi, *ma, links, 0.05, periodic=7)
+    pkg.fused_trt_libb_v2_step_3d_(b, fi, *mb, solid, qw, *uw, Nx, Ny, Nz, 0.05,
+                                   periodic=(True, True, True))
+    assert torch.equal(a, b) and all(torch.equal(x, y) for x, y in zip(ma, mb))
+    links.close()
+
+
 @pytest.mark.parametrize("size", [(2, 2), (2, 3), (16, 13), (130, 9), (256, 3), (258, 5)])
 @pytest.mark.parametrize("vt", [False, True])
 def test_natconv_pairs_match_one_node(cuda, pkg, size, vt):
