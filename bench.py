@@ -785,7 +785,7 @@ def bench_batch(pkg, n_cases=256, max_steps=50000, check_every=100, tol=1e-6, st
     log-uniform [100, 2000], u_lid=0.1, one persistent launch per rank (the
     cases are split across ranks with no data exchange), replayed from a
     captured CUDA graph (graph=True).  autotune: the schedule is tuned first,
-    and the tuned and the fixed schedules' throughputs are
+    and the tuned and the untuned (fixed) schedules' throughputs are
     reported.  With error_cases > 0, that many cases (spread over the size
     range) are rerun on the FP64 reference-arithmetic MRT cavity step for the
     same number of steps and their velocity error is reported; every case that
@@ -836,7 +836,7 @@ def bench_batch(pkg, n_cases=256, max_steps=50000, check_every=100, tol=1e-6, st
            "steps_min_median_max": [int(min(steps)), int(np.median(steps)), int(max(steps))]}
     if tune:
         tune["tuned_over_fixed"] = round(tune["best_mlups"] / tune["fixed_mlups"], 3)
-        tune["fixed_schedule"] = "256-node tiles dealt out one by one, blocks per SM at the occupancy limit"
+        tune["fixed_schedule"] = "256-node tiles, blocks per SM at the occupancy limit (untuned default)"
         out["autotune"] = tune
     if rank == 0:
         nonfinite = []

@@ -558,9 +558,9 @@ int kb_batch_destroy(kb_batch *b);
 int kb_batch_reset(kb_batch *b, void *stream);
 /* Queue the run (asynchronous, one cooperative launch).  check_every >= 2;
  * max_steps a multiple of check_every; tile_nodes (multiple of 32) and
- * blocks_per_sm <= 0 take the autotuned choice.  Untuned, tile_nodes <= 0
- * gives each block one run of consecutive 256-node tiles and blocks_per_sm <= 0
- * the occupancy limit; a tile size deals the tiles out one by one. */
+ * blocks_per_sm <= 0 take the autotuned choice (else 256 / occupancy).  Tiles
+ * of up to 256 nodes are shared out in runs of consecutive tiles, one run per
+ * block, longer ones one by one. */
 int kb_batch_run(kb_batch *b, int max_steps, int check_every, double tol, int tile_nodes,
                  int blocks_per_sm, void *stream);
 /* Node updates done, live tiles left and the grid-barrier timeout flag
@@ -573,10 +573,10 @@ int kb_batch_case(kb_batch *b, int c, int *N, int *steps, double *residual, int 
                   float *ux_host, float *uy_host, void *stream);
 /* Time trial_steps of every (tile_nodes, blocks_per_sm) candidate (tiles of
  * 256 ... 4096 nodes, 1 ... the occupancy limit of blocks per SM), keep the
- * fastest of them and of the untuned schedule for later runs; reports its
- * MLUPS (the untuned schedule as 256 nodes at the occupancy limit) and that of
- * the fixed schedule 256-node tiles, as many blocks per SM as fit.  Resets the
- * batch. */
+ * fastest for later runs; reports its MLUPS and that of the fixed schedule
+ * kb_batch_run takes untuned (256-node tiles, as many blocks per SM as fit).
+ * The reported pair passed to kb_batch_run selects the same schedule.  Resets
+ * the batch. */
 int kb_batch_autotune(kb_batch *b, int trial_steps, int *best_tile, int *best_bpsm,
                       double *best_mlups, double *fixed_mlups, void *stream);
 /* Device pointer to case c's final populations (9 planes of N*N, storage

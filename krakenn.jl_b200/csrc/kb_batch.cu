@@ -13,11 +13,12 @@
 // Schedule: the nodes of all active cases are cut into tiles of `tile_nodes`
 // consecutive nodes of one case.  The kernel is launched cooperatively with
 // blocks_per_sm x SMs blocks; each step the blocks share the active tile list
-// (untuned: equal runs of consecutive 256-node tiles, which balances to one
-// tile and keeps a block in one case: 48 cavities of 64^2 to 512^2 in FP16 ran
-// at 106 GLUPS against 64 with every nblocks-th tile; tuned or given a tile
-// size: every nblocks-th tile), then meet at a grid barrier (spin bounded by an iteration
-// limit; a timeout sets an error flag that every block sees and returns on).
+// (tiles of up to 256 nodes, the untuned size among them, in equal runs of
+// consecutive tiles, which balances to one tile and keeps a block in one case:
+// 48 cavities of 64^2 to 512^2 in FP16 ran at 105 GLUPS against 63 with every
+// nblocks-th tile; longer tiles every nblocks-th), then meet at a grid barrier
+// (spin bounded by an iteration limit; a timeout sets an error flag that every
+// block sees and returns on).
 // Every `check_every` steps the residual of each case is reduced on the device
 // (FP64 atomics per tile), block 0 retires converged / finished / non-finite
 // cases and compacts the tile list, and the next step runs only live tiles.
@@ -713,11 +714,16 @@ int kb_batch_run(kb_batch *b, int max_steps, int check_every, double tol, int ti
     KB_REQUIRE(check_every >= 2, "kb_batch_run: check_every must be >= 2");
     KB_REQUIRE(max_steps >= check_every && max_steps % check_every == 0,
                "kb_batch_run: max_steps must be a positive multiple of check_every");
-    const bool ranges = tile_nodes <= 0 && b->tuned_tile <= 0;
     if (tile_nodes <= 0) tile_nodes = b->tuned_tile > 0 ? b->tuned_tile : 256;
     if (blocks_per_sm <= 0) blocks_per_sm = b->tuned_bpsm > 0 ? b->tuned_bpsm : 0;
     KB_REQUIRE(tile_nodes % 32 == 0 && tile_nodes <= (1 << 20),
                "kb_batch_run: tile_nodes must be a multiple of 32");
+    // Tiles of up to 256 nodes are shared out in runs, longer ones one by one.
+    // GLUPS in runs and one by one: 256 nodes, FP16, 48 cases of 64^2 to 512^2
+    // 107 and 63, odd sizes 70 and 58, 200 cases of 64^2 and 96^2 93 and 67,
+    // FP32 66 and 56; but 512 nodes, FP32 69 and 77, and 4096 nodes, FP16, 256
+    // cases 118 and 122.
+    const bool ranges = tile_nodes <= 256;
     cudaStream_t s = kb::as_stream(stream);
     if (tile_nodes != b->tile_nodes) {
         if (int r = build_tiles(b, tile_nodes)) return r;
@@ -782,17 +788,20 @@ int kb_batch_autotune(kb_batch *b, int trial_steps, int *best_tile, int *best_bp
     KB_REQUIRE(b, "kb_batch_autotune: null handle");
     KB_REQUIRE(trial_steps >= 2 && trial_steps % 2 == 0, "kb_batch_autotune: trial_steps must be even and >= 2");
     cudaStream_t s = kb::as_stream(stream);
-    // the candidates: tile sizes x every residency up to the occupancy limit
-    // (the fixed schedule they are compared with: 256-node tiles, as many
-    // blocks per SM as fit), and the untuned schedule
+    // the candidates: tile sizes x every residency up to the occupancy limit;
+    // the fixed schedule is what kb_batch_run takes untuned (256-node tiles,
+    // as many blocks per SM as fit)
     const int occ = batch_occupancy(b->dtype);
     if (occ < 1) return kb::set_error(KB_ERR_UNSUPPORTED, "kb_batch_autotune: kernel does not fit an SM");
     const int tiles[] = {256, 512, 1024, 2048, 4096};
     double best = -1.0, fixed = -1.0;
     int bt = 256, bb = occ;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
+    struct Event {
+        cudaEvent_t e = nullptr;
+        Event() { cudaEventCreate(&e); }
+        ~Event() { cudaEventDestroy(e); }
+        operator cudaEvent_t() const { return e; }
+    } e0, e1;
     for (int tn : tiles)
         for (int bp = 1; bp <= occ; ++bp) {
             if (int r = build_tiles(b, tn)) return r;
@@ -811,29 +820,8 @@ int kb_batch_autotune(kb_batch *b, int trial_steps, int *best_tile, int *best_bp
             if (tn == 256 && bp == occ) fixed = mlups;
             if (mlups > best) { best = mlups; bt = tn; bb = bp; }
         }
-    // the untuned schedule (ranges of the 256-node list at the occupancy limit)
-    bool ranges = false;
-    {
-        b->tuned_tile = b->tuned_bpsm = 0;
-        if (int r = build_tiles(b, 256)) return r;
-        if (int r = reset(b, s)) return r;
-        cudaEventRecord(e0, s);
-        if (int r = kb_batch_run(b, trial_steps, trial_steps, 0.0, 0, 0, stream)) return r;
-        cudaEventRecord(e1, s);
-        cudaError_t e = cudaEventSynchronize(e1);
-        if (e != cudaSuccess) return cuda_err("kb_batch_autotune", e);
-        long long up = 0;
-        int live = 0, tout = 0;
-        if (int r = kb_batch_status(b, &up, &live, &tout, stream)) return r;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        const double mlups = (double)up / (ms * 1e-3) / 1e6;
-        if (mlups > best) { best = mlups; bt = 256; bb = occ; ranges = true; }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    b->tuned_tile = ranges ? 0 : bt;
-    b->tuned_bpsm = ranges ? 0 : bb;
+    b->tuned_tile = bt;
+    b->tuned_bpsm = bb;
     if (int r = build_tiles(b, bt)) return r;
     if (int r = reset(b, s)) return r;
     if (best_tile) *best_tile = bt;

@@ -55,3 +55,24 @@ def test_sweep_mass_does_not_drift(cuda, pkg, N):
         x, y = y, x
     assert abs(out.value - pkg.ops.mass(x)) / (N * N) < 1e-6
     b.close()
+
+
+def test_reported_schedules_can_be_asked_for(cuda, pkg):
+    """A (tile_nodes, blocks_per_sm) pair names one schedule: the untuned one
+    is 256-node tiles at the occupancy limit, so asking for that pair takes its
+    time (dealing such tiles out one by one takes 1.7 times as long)."""
+    import torch
+    N, nu, u, _ = pkg.sweep_cases(48, seed=3)
+    b = pkg.CavityBatch(N, nu, u, "f16")
+    took = {}
+    for tn in (0, 256, 0, 256):
+        for _ in range(3):
+            b.reset()
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            b.run(max_steps=200, check_every=100, tol=0.0, tile_nodes=tn)
+            e[1].record()
+            torch.cuda.synchronize()
+            took[tn] = min(took.get(tn, 1e9), e[0].elapsed_time(e[1]))
+    assert took[256] < 1.25 * took[0]
+    b.close()
