@@ -11,6 +11,7 @@ src/kernels/persistent_bgk_2d.jl:160).
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -126,30 +127,64 @@ class CavityBatch:
                     fixed_mlups=fixed.value)
 
 
+# Streams between two captures, as (device, stream); making and destroying one
+# per capture took 80 us of a driver run.  At most _IDLE_MOST are kept.
+_idle: list = []
+_IDLE_MOST = 8
+_idle_lock = threading.Lock()
+
+
+def _take_stream():
+    dev = torch.cuda.current_device()
+    with _idle_lock:
+        for i, (d, s) in enumerate(_idle):
+            if d == dev:
+                del _idle[i]
+                return s
+    p = C.c_void_p()
+    call("kb_stream_create", C.byref(p))
+    return torch.cuda.ExternalStream(p.value)
+
+
+def _give_back(stream):
+    with _idle_lock:
+        if len(_idle) < _IDLE_MOST:
+            _idle.append((stream.device.index, stream))
+            return
+    call("kb_stream_destroy", C.c_void_p(stream.cuda_stream))
+
+
 class Graph:
-    """Capture library calls issued on a stream of its own, then replay them.
-    The stream is not one of torch's pool, which hands the same 32 streams out
-    in turn: another thread's work queued on a pool stream while a graph
-    captures on it would be captured instead of run."""
+    """Capture library calls, then replay them.  While it captures, a graph has
+    a stream of its own (`stream`, the current stream inside the `with`).  It is
+    not one of torch's pool, which hands the same 32 streams out in turn:
+    another thread's work queued on a pool stream while a graph captures on it
+    would be captured instead of run."""
 
     def __init__(self):
         self._g = C.c_void_p()
-        self._s = C.c_void_p()
-        call("kb_stream_create", C.byref(self._s))
-        self.stream = torch.cuda.ExternalStream(self._s.value)
+        self.stream = None
 
     def __enter__(self):
-        self.stream.wait_stream(torch.cuda.current_stream())
-        call("kb_graph_begin", self._s)
-        self._ctx = torch.cuda.stream(self.stream)
+        stream = _take_stream()
+        try:
+            stream.wait_stream(torch.cuda.current_stream())
+            call("kb_graph_begin", C.c_void_p(stream.cuda_stream))
+        except BaseException:
+            _give_back(stream)
+            raise
+        self.stream = stream
+        self._ctx = torch.cuda.stream(stream)
         self._ctx.__enter__()
         return self
 
     def __exit__(self, *exc):
+        stream, self.stream = self.stream, None
         try:
-            call("kb_graph_end", self._s, C.byref(self._g))
+            call("kb_graph_end", C.c_void_p(stream.cuda_stream), C.byref(self._g))
         finally:
             self._ctx.__exit__(*exc)
+            _give_back(stream)
         return False
 
     def launch(self):
@@ -159,9 +194,6 @@ class Graph:
         if self._g:
             call("kb_graph_destroy", self._g)
             self._g = C.c_void_p()
-        if self._s:
-            call("kb_stream_destroy", self._s)
-            self._s = C.c_void_p()
 
     def __del__(self):
         try:

@@ -8,15 +8,27 @@ pytestmark = pytest.mark.gpu
 
 
 def test_capture_stream_is_not_a_pool_stream(cuda, pkg):
+    """More streams at once than are kept between captures; they go back and
+    are taken again."""
+    b = pkg.batch
     pool = {torch.cuda.Stream().cuda_stream for _ in range(64)}
-    graphs = [pkg.Graph() for _ in range(33)]
-    own = [g.stream.cuda_stream for g in graphs]
-    assert len(set(own)) == len(own) and not pool & set(own)
-    for g in graphs:
-        g.close()
+    taken = [b._take_stream() for _ in range(b._IDLE_MOST + 3)]
+    own = {s.cuda_stream for s in taken}
+    assert len(own) == len(taken) and not pool & own
+    for s in taken:
+        b._give_back(s)
+    assert len(b._idle) == b._IDLE_MOST
+    g = pkg.Graph()
+    with g:
+        assert g.stream.cuda_stream in own
+        assert torch.cuda.current_stream().cuda_stream == g.stream.cuda_stream
+        assert len(b._idle) == b._IDLE_MOST - 1
+    assert len(b._idle) == b._IDLE_MOST
+    g.close()
 
 
 def test_failed_begin_leaves_the_current_stream(cuda, pkg, monkeypatch):
+    pkg.batch._give_back(pkg.batch._take_stream())
     g = pkg.Graph()
     before = torch.cuda.current_stream().cuda_stream
 
