@@ -9,10 +9,14 @@
 // beside the value.  A reader polls its packet until the number is the step's:
 // no fence and no barrier between blocks, one write and one read of L2.
 //
-// One B200, us per step, captured launches -> this: 32^2 FP64 1.87 -> 1.41,
-// 128^2 1.88 -> 1.47, 256^2 2.78 -> 1.79; FP32 2.01 -> 1.24, 1.88 -> 1.42, 2.40
-// -> 1.68, 384 x 256 2.63 -> 2.01.  It wins at every size that is resident, so
-// that is the rule.  At 128^2 FP64, tiles of 32 x 4 and 128 x 1 took 4 % longer.
+// One B200, us per step, captured launches -> this: 32^2 FP64 1.67 -> 1.42,
+// 128^2 1.67 -> 1.47, 256^2 2.57 -> 1.79; FP32 1.67 -> 1.27, 1.67 -> 1.42, 2.18
+// -> 1.68, 384 x 256 (about the largest that is resident) 2.46 -> 2.02.  Narrow
+// grids, FP64: 1 x 512 1.41 -> 1.19, 24 x 512 1.67 -> 1.34, 65 x 300 (tiles of
+// 33 nodes) 1.80 -> 1.53, 65 x 512 1.93 -> 1.73, 1024 x 16 1.68 -> 1.50; the
+// least gain of 48 grids in both precisions and with both lids is 6 % (65 x 300
+// FP32, moving lid).  It wins at every resident size, so that is the rule.
+// At 128^2 FP64, tiles of 32 x 4 and 128 x 1 took 4 % longer.
 // Packets fetched by warps of their own (20 % longer), or read again by the
 // whole row until all are in (25 %), load L2 with more polls and lose; so does
 // a pair of thermal lattices, whose step has twice the packets (256 x 64: 2.0 us

@@ -36,8 +36,9 @@ def test_sweep_mass_does_not_drift(cuda, pkg, N):
     """Rest population from conservation: the mass of an FP32 cavity stays at
     rest's to the rounding of the stores.  10 000 steps of N^2 nodes round 9
     deviations of at most 0.1 w_q each to 2^-24: a random walk of 3e-9 per
-    node and 1e-4 steps^-1/2; 1e-7 per node bounds it with room, while a
-    coefficient error of half an ulp per step would reach 1e-5."""
+    node and 1e-4 steps^-1/2 (measured: 5e-9 and 1.5e-8); 1e-7 per node bounds
+    it with room, while a coefficient error of half an ulp per step would reach
+    1e-5."""
     import ctypes as C
     import torch
     b = pkg.CavityBatch(np.array([N], np.int32), np.array([0.05]), np.array([0.1]), "f32")
@@ -53,7 +54,7 @@ def test_sweep_mass_does_not_drift(cuda, pkg, N):
     for _ in range(10000):
         pkg.cavity_mrt_step_2d_(y, x, None, None, None, None, N, N, 0.05, 0.1)
         x, y = y, x
-    assert abs(out.value - pkg.ops.mass(x)) / (N * N) < 1e-6
+    assert abs(out.value - pkg.ops.mass(x)) / (N * N) < 1e-7
     b.close()
 
 
